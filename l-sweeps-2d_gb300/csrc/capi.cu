@@ -54,7 +54,7 @@ struct lsw_ctx {
   int max_nx = 0, max_ny = 0, ncell = 0;
   long long LP = 0;
   std::vector<DevCell> cells;
-  DevBuf d_cells, d_prof, d_gprof, d_m, d_fac, d_work, d_status;
+  DevBuf d_symt, d_cells, d_prof, d_gprof, d_m, d_fac, d_work, d_status;
   // per batch size
   std::map<int, std::unique_ptr<Schedule>> sched;
   std::map<int, std::unique_ptr<DevBuf[]>> sched_bufs;
@@ -171,19 +171,14 @@ lsw_status cuda_fail(lsw_ctx* c, cudaError_t e, const char* where) {
 inline size_t csize(int prec) { return prec == LSW_PREC_C128 ? 16 : 8; }
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
-DevCell make_cell(int I, int J, int N, int m, int p, bool split) {
+DevCell make_cell(int I, int J, int N, int m, int p, bool sym) {
   DevCell c{};
   const DirGeom gx = dir_geom(J, N, m, p), gy = dir_geom(I, N, m, p);
   c.I = I; c.J = J;
   c.nx = gx.nd; c.ny = gy.nd;
   c.lox = gx.lo; c.loy = gy.lo;
   c.ldn = (gy.nd + 3) & ~3;
-  // bf16-split factors: a column stride of 4 (mod 8) complex values keeps the
-  // four columns of an mma A fragment in distinct shared-memory banks
-  if (split) {
-    c.ldn = gy.nd;
-    while (c.ldn % 8 != 4) ++c.ldn;
-  }
+  c.blk = sym ? SymTiles::elems(gy.nd) : c.ny * c.ldn;
   for (int s = 0; s < 2; ++s) {
     for (int l = 0; l < 4; ++l) { c.lx[s][l] = gx.lines[s][l]; c.ly[s][l] = gy.lines[s][l]; }
     c.ownx[s][0] = gx.own[s][0]; c.ownx[s][1] = gx.own[s][1];
@@ -201,6 +196,38 @@ void fill_info(const DevCell& c, lsw_cell_info* o) {
   }
 }
 
+// whether the factors are in symmetric tiles: complex64 (but for contexts that
+// run or tune tensor-core line products, which need whole columns) and split
+bool sym_factors(const lsw_ctx* c) {
+  return c->prec == LSW_PREC_SPLIT || (c->prec == LSW_PREC_C64 && !c->sweep_tc && !c->force_tc);
+}
+int fit_mask(const lsw_ctx* c, int slots) {
+  return sym_factors(c) ? sym_fit_mask(c->prec == LSW_PREC_SPLIT, c->max_ny, c->max_nx, slots)
+                        : front_fit_mask(c->prec == LSW_PREC_C128, c->max_ny, c->max_nx, slots);
+}
+cudaError_t run_front(const lsw_ctx* c, const FrontArgs& a, cudaStream_t st) {
+  if (sym_factors(c)) return launch_front_sym(a, c->max_ny, c->max_nx, st);
+  return c->prec == LSW_PREC_C128 ? launch_front<double>(a, c->max_ny, c->max_nx, st)
+                                  : launch_front<float>(a, c->max_ny, c->max_nx, st);
+}
+
+// The diagonal scaling that makes the y-couplings symmetric, e_0 = 1,
+// (e_j / e_{j-1})^2 = lo_j / hi_{j-1}: off_j = lo_j e_{j-1} / e_j couples j and
+// j - 1 both ways.  (lo, hi of the interior are equal, those of the PML of like
+// size, so e stays near 1.)
+void push_symmetrised(std::vector<double2>& v, const Profile1D& pr) {
+  const size_t n = pr.lo_re.size();
+  std::vector<cplx> off(n), e(n, cplx(1.0, 0.0));
+  for (size_t j = 1; j < n; ++j) {
+    const cplx lo(pr.lo_re[j], pr.lo_im[j]), hi(pr.hi_re[j - 1], pr.hi_im[j - 1]);
+    const cplx r = std::sqrt(lo / hi);
+    e[j] = e[j - 1] * r;
+    off[j] = lo / r;
+  }
+  for (const cplx& q : off) v.push_back(make_double2(q.real(), q.imag()));
+  for (const cplx& q : e) v.push_back(make_double2(q.real(), q.imag()));
+}
+
 void push_profile(std::vector<double2>& v, const Profile1D& pr) {
   const size_t n = pr.lo_re.size();
   for (size_t i = 0; i < n; ++i) v.push_back(make_double2(pr.lo_re[i], pr.lo_im[i]));
@@ -209,7 +236,7 @@ void push_profile(std::vector<double2>& v, const Profile1D& pr) {
 }
 
 size_t device_bytes(const lsw_ctx* c) {
-  size_t b = c->d_cells.bytes + c->d_prof.bytes + c->d_gprof.bytes + c->d_m.bytes + c->d_fac.bytes +
+  size_t b = c->d_symt.bytes + c->d_cells.bytes + c->d_prof.bytes + c->d_gprof.bytes + c->d_m.bytes + c->d_fac.bytes +
              c->d_work.bytes + c->d_status.bytes + c->d_traces.bytes + c->d_outs.bytes + c->d_scratch.bytes +
              c->k_basis.bytes + c->k_zbasis.bytes + c->k_tmp.bytes + c->k_tmp2.bytes + c->k_r.bytes +
              c->k_part.bytes + c->k_small.bytes + c->k_small2.bytes + c->k_nrm.bytes + c->ls_items.bytes +
@@ -220,12 +247,13 @@ size_t device_bytes(const lsw_ctx* c) {
   return b;
 }
 
-// CTAs per half for a single-cell solve: `cl`, or the next larger size whose
-// launch fits in shared memory
+// CTAs per half for a single-cell solve: `cl`, or the next larger, else the
+// next smaller size whose launch fits in shared memory
 int fitting_cluster(const lsw_ctx* ctx, int slots, int cl) {
-  const int mask = front_fit_mask(ctx->prec == LSW_PREC_C128, ctx->prec == LSW_PREC_SPLIT, ctx->max_ny,
-                                  ctx->max_nx, slots);
+  const int mask = fit_mask(ctx, slots);
   for (int c = cl; c <= 4; c *= 2)
+    if (mask & (1 << c)) return c;
+  for (int c = cl / 2; c >= 1; c /= 2)
     if (mask & (1 << c)) return c;
   return cl;   // nothing fits: the launch reports it
 }
@@ -241,9 +269,11 @@ FrontPlan base_plan(const lsw_ctx* ctx) {
     // tensor-core matvec: the per-column cost hardly grows with the slots
     plan.line_overhead = 2200.0; plan.slot_cost = 0.0; plan.col_cost = 40.0; plan.col_slot_cost = 3.0;
   }
-  for (int cl = 1; cl <= 4; cl *= 2) plan.max_clusters[cl] = front_max_clusters(dbl, 2 * cl);
-  for (int r = 1; r <= 16; ++r)
-    plan.fit_mask[r] = front_fit_mask(dbl, ctx->prec == LSW_PREC_SPLIT, ctx->max_ny, ctx->max_nx, r);
+  plan.sym = sym_factors(ctx);
+  for (int cl = 1; cl <= 4; cl *= 2)
+    plan.max_clusters[cl] = plan.sym ? sym_max_clusters(ctx->prec == LSW_PREC_SPLIT, 2 * cl)
+                                     : front_max_clusters(dbl, 2 * cl);
+  for (int r = 1; r <= 16; ++r) plan.fit_mask[r] = fit_mask(ctx, r);
   if (plan.max_clusters[1] <= 0) plan.max_clusters[1] = ctx->nsm / 2;
   plan.tc_scratch = ctx->prec == LSW_PREC_C64 && (ctx->sweep_tc || ctx->force_tc);
   return plan;
@@ -300,7 +330,7 @@ struct TuneEntry {
 bool tc_candidates(const lsw_ctx* ctx) { return ctx->prec == LSW_PREC_C64 && ctx->sweep_tc; }
 bool tc_fits(const lsw_ctx* ctx, int max_slots, int cl) {
   if (ctx->prec != LSW_PREC_C64 || max_slots < 1 || max_slots > 16) return false;
-  return (front_fit_mask(false, false, ctx->max_ny, ctx->max_nx, front_tc_slots(max_slots), true) >> cl) & 1;
+  return (front_fit_mask(false, ctx->max_ny, ctx->max_nx, front_tc_slots(max_slots), true) >> cl) & 1;
 }
 std::mutex g_tune_mu;
 std::map<std::string, TuneEntry> g_tune_cache;
@@ -596,6 +626,7 @@ lsw_status launch_front_of(lsw_ctx* ctx, const Schedule* sc, size_t fi, cudaStre
   a.n_dof = ctx->n_dof; a.N = ctx->N; a.m = ctx->m; a.p = ctx->p;
   a.err = ctx->d_status.as<int>() + 1;
   a.wait_cycles = ctx->wait_cycles;
+  a.symt = ctx->d_symt.as<SymTable>();
   a.split = ctx->prec == LSW_PREC_SPLIT ? 1 : 0;
   const Front& f = sc->fronts[fi];
   if (i1 < 0) i1 = f.item_count;
@@ -605,9 +636,7 @@ lsw_status launch_front_of(lsw_ctx* ctx, const Schedule* sc, size_t fi, cudaStre
   a.max_slots = f.max_slots;
   a.cluster = f.cluster;
   a.tc = f.tc ? 1 : 0;
-  cudaError_t e = ctx->prec != LSW_PREC_C128 ? launch_front<float>(a, ctx->max_ny, ctx->max_nx, st)
-                                             : launch_front<double>(a, ctx->max_ny, ctx->max_nx, st);
-  CK(e, "front kernel");
+  CK(run_front(ctx, a, st), "front kernel");
   return LSW_OK;
 }
 
@@ -877,6 +906,27 @@ namespace {
 constexpr size_t kNoAllocScratchBytes = size_t(8) << 20;   // 8 MiB
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
+// scratch of a single-cell solve: elements of an item, bytes of the descriptors
+long long local_item_scratch(const lsw_ctx* ctx, const DevCell& cl, int nrhs, int clus) {
+  return item_scratch(cl, front_rpad(std::min(front_rmax(ctx->prec == LSW_PREC_C128), nrhs)), clus, sym_factors(ctx));
+}
+size_t local_desc_bytes(int nrhs, int rmax) {
+  const size_t items = (nrhs + rmax - 1) / rmax;
+  return (items * sizeof(DevItem) + (size_t)nrhs * sizeof(DevSlot) + 255) & ~size_t(255);
+}
+// CTAs per half of a single-cell solve, the same with and without allocation:
+// one where the x_k rows that several CTAs need would take the scratch past the
+// fixed array
+int local_cluster(const lsw_ctx* ctx, const DevCell& cl, int nrhs) {
+  const int rmax = front_rmax(ctx->prec == LSW_PREC_C128), items = (nrhs + rmax - 1) / rmax;
+  int c = fitting_cluster(ctx, std::min(rmax, nrhs), front_cluster(items, ctx->nsm, ctx->max_cluster));
+  if (sym_factors(ctx) && c > 1 &&
+      local_desc_bytes(nrhs, rmax) + (size_t)items * local_item_scratch(ctx, cl, nrhs, c) * csize(ctx->prec) >
+          kNoAllocScratchBytes)
+    c = fitting_cluster(ctx, std::min(rmax, nrhs), 1);
+  return c;
+}
+
 // writes the descriptors of `nrhs` full-cell right-hand sides of one cell:
 // items of at most rmax slots, each with its share of the forward storage
 __global__ void k_noalloc_desc(DevItem* items, DevSlot* slots, int cell, int nrhs, int rmax,
@@ -1115,13 +1165,15 @@ lsw_status lsw_problem_setup(lsw_ctx* ctx, const lsw_geom* g, const double* m_gr
   ctx->max_nx = ctx->max_ny = 0;
   for (int I = 0; I < ctx->N; ++I)
     for (int J = 0; J < ctx->N; ++J) {
-      DevCell c = make_cell(I, J, ctx->N, ctx->m, ctx->p, precision == LSW_PREC_SPLIT);
+      DevCell c = make_cell(I, J, ctx->N, ctx->m, ctx->p, sym_factors(ctx));
       c.fac_off = fac_off;
-      fac_off += (long long)c.nx * c.ny * c.ldn;
+      fac_off += (long long)c.nx * c.blk;
       c.prof_off = (long long)prof.size();
       const DirGeom gx = dir_geom(J, ctx->N, ctx->m, ctx->p), gy = dir_geom(I, ctx->N, ctx->m, ctx->p);
       push_profile(prof, make_profile(gx.nel, ctx->p, ctx->h, ctx->C));
-      push_profile(prof, make_profile(gy.nel, ctx->p, ctx->h, ctx->C));
+      const Profile1D prof_y = make_profile(gy.nel, ctx->p, ctx->h, ctx->C);
+      push_profile(prof, prof_y);
+      push_symmetrised(prof, prof_y);
       ctx->max_nx = std::max(ctx->max_nx, c.nx);
       ctx->max_ny = std::max(ctx->max_ny, c.ny);
       ctx->cells.push_back(c);
@@ -1136,8 +1188,13 @@ lsw_status lsw_problem_setup(lsw_ctx* ctx, const lsw_geom* g, const double* m_gr
   CK(ctx->d_m.ensure((size_t)ctx->n2 * sizeof(double)), "cudaMalloc(m)");
   CK(ctx->d_fac.ensure((size_t)fac_off * cs), "cudaMalloc(factors)");
   CK(ctx->d_status.ensure(16), "cudaMalloc(status)");
-  if (precision == LSW_PREC_SPLIT) {
-    // the previous FP32 Schur-complement inverse of each cell's two half
+  if (!ctx->d_symt.p) {
+    static const SymTable symt;
+    CK(ctx->d_symt.ensure(sizeof(SymTable)), "cudaMalloc(tile order)");
+    CK(cudaMemcpy(ctx->d_symt.p, &symt, sizeof(SymTable), cudaMemcpyHostToDevice), "H2D tile order");
+  }
+  if (sym_factors(ctx)) {
+    // the previous whole FP32 Schur-complement inverse of each cell's two half
     // chains, for the recurrences and the middle line
     CK(ctx->d_work.ensure((size_t)2 * ctx->ncell * ctx->max_ny * (ctx->max_ny + 8) * sizeof(float2)),
        "cudaMalloc(factor work)");
@@ -1180,21 +1237,20 @@ lsw_status lsw_factorize(lsw_ctx* ctx, void* stream) {
   CK(cudaMemsetAsync(ctx->d_status.p, 0, 16, st), "memset status");
   ctx->launches += 2;   // half chains, middle lines
   const double w2 = ctx->omega * ctx->omega;
+  const int layout = !sym_factors(ctx) ? FL_WHOLE : ctx->prec == LSW_PREC_SPLIT ? FL_SYM_SPLIT : FL_SYM;
   const bool tc = ctx->prec != LSW_PREC_C128 && ctx->factor_tc && factorize_tc_supported(ctx->max_ny);
   cudaError_t e = tc ? launch_factorize_tc(ctx->d_cells.as<DevCell>(), ctx->ncell, ctx->d_prof.as<double2>(),
                                            ctx->d_m.as<double>(), ctx->n_dof, w2, ctx->d_fac.p, ctx->d_work.p,
-                                           ctx->max_ny, ctx->d_status.as<int>(), st, ctx->prec == LSW_PREC_SPLIT,
-                                           ctx->wait_cycles)
+                                           ctx->max_ny, ctx->d_status.as<int>(), st, layout, ctx->wait_cycles, ctx->d_symt.as<SymTable>())
                   : ctx->prec != LSW_PREC_C128
                       ? launch_factorize<float>(ctx->d_cells.as<DevCell>(), ctx->ncell, ctx->d_prof.as<double2>(),
                                                 ctx->d_m.as<double>(), ctx->n_dof, w2, ctx->d_fac.p, ctx->d_work.p,
-                                                ctx->max_ny, ctx->d_status.as<int>(), st, ctx->prec == LSW_PREC_SPLIT,
-                                                ctx->factor_lookahead, ctx->wait_cycles)
+                                                ctx->max_ny, ctx->d_status.as<int>(), st, layout, ctx->factor_lookahead, ctx->wait_cycles, ctx->d_symt.as<SymTable>())
                       : launch_factorize<double>(ctx->d_cells.as<DevCell>(), ctx->ncell, ctx->d_prof.as<double2>(),
                                                  ctx->d_m.as<double>(), ctx->n_dof, w2, ctx->d_fac.p, ctx->d_work.p,
-                                                 ctx->max_ny, ctx->d_status.as<int>(), st, false,
+                                                 ctx->max_ny, ctx->d_status.as<int>(), st, layout,
                                                  false,   // complex128: the update dominates, no overlap
-                                                 ctx->wait_cycles);
+                                                 ctx->wait_cycles, nullptr);
   CK(e, "factorize kernel");
   int status = 0;
   CK(cudaMemcpyAsync(&status, ctx->d_status.p, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H status");
@@ -1275,7 +1331,7 @@ lsw_status lsw_apply_precond_profiled(lsw_ctx* ctx, const void* x, void* y, int 
   for (const Front& fr : sc->fronts) {
     for (int i = fr.item_begin; i < fr.item_begin + fr.item_count; ++i) {
       const DevCell& c = ctx->cells[items[i].cell];
-      streamed += 2.0 * (double)c.nx * c.ny * c.ldn * cs + 4.0 * items[i].slot_count * (double)c.nx * c.ny * cs;
+      streamed += 2.0 * (double)c.nx * c.blk * cs + 4.0 * items[i].slot_count * (double)c.nx * c.ny * cs;
     }
   }
   prof->fronts = (int)sc->fronts.size();
@@ -1327,12 +1383,13 @@ lsw_status lsw_local_solve(lsw_ctx* ctx, int cell, const void* b, void* x, int n
   std::vector<DevItem> items;
   std::vector<DevSlot> slots;
   long long scr = 0;
+  const int clus = local_cluster(ctx, cl, nrhs);
   for (int r0 = 0; r0 < nrhs; r0 += rmax) {
     DevItem it{};
     it.cell = cell; it.slot_begin = (int)slots.size(); it.group_begin = 0; it.group_count = 0;
     it.slot_count = std::min(rmax, nrhs - r0);
     it.scratch_off = scr;
-    scr += (long long)(cl.nx + 1) * front_rpad(it.slot_count) * cl.ny;
+    scr += item_scratch(cl, front_rpad(it.slot_count), clus, sym_factors(ctx));
     for (int r = r0; r < r0 + it.slot_count; ++r) {
       DevSlot s{};
       s.kind = SK_CELLVEC; s.rhs = r;
@@ -1364,10 +1421,10 @@ lsw_status lsw_local_solve(lsw_ctx* ctx, int cell, const void* b, void* x, int n
   a.max_slots = std::min(rmax, nrhs);
   a.err = ctx->d_status.as<int>() + 1;
   a.wait_cycles = ctx->wait_cycles;
+  a.symt = ctx->d_symt.as<SymTable>();
   a.split = ctx->prec == LSW_PREC_SPLIT ? 1 : 0;
-  a.cluster = fitting_cluster(ctx, a.max_slots, front_cluster(a.item_count, ctx->nsm, ctx->max_cluster));
-  cudaError_t e = dbl ? launch_front<double>(a, ctx->max_ny, ctx->max_nx, st) : launch_front<float>(a, ctx->max_ny, ctx->max_nx, st);
-  CK(e, "local solve kernel");
+  a.cluster = clus;
+  CK(run_front(ctx, a, st), "local solve kernel");
   ctx->launches += 1;
   return check_kernel_err(ctx, st);
 }
@@ -1784,8 +1841,9 @@ lsw_status lsw_local_solve_noalloc(lsw_ctx* ctx, int cell, const void* b, void* 
   const int rmax = front_rmax(dbl);
   const DevCell& cl = ctx->cells[cell];
   const int n_items = (nrhs + rmax - 1) / rmax;
-  const long long per_item = (long long)(cl.nx + 1) * front_rpad(std::min(rmax, nrhs)) * cl.ny;
-  const size_t desc_bytes = ((size_t)n_items * sizeof(DevItem) + (size_t)nrhs * sizeof(DevSlot) + 255) & ~size_t(255);
+  const int clus = local_cluster(ctx, cl, nrhs);
+  const long long per_item = local_item_scratch(ctx, cl, nrhs, clus);
+  const size_t desc_bytes = local_desc_bytes(nrhs, rmax);
   const size_t need = desc_bytes + (size_t)n_items * per_item * csize(ctx->prec);
   if (need > kNoAllocScratchBytes) {
     return fail(ctx, LSW_ERR_INVALID_ARGUMENT,
@@ -1821,10 +1879,10 @@ lsw_status lsw_local_solve_noalloc(lsw_ctx* ctx, int cell, const void* b, void* 
   a.max_slots = std::min(rmax, nrhs);
   a.err = ctx->d_status.as<int>() + 1;
   a.wait_cycles = ctx->wait_cycles;
+  a.symt = ctx->d_symt.as<SymTable>();
   a.split = ctx->prec == LSW_PREC_SPLIT ? 1 : 0;
-  a.cluster = fitting_cluster(ctx, a.max_slots, front_cluster(a.item_count, ctx->nsm, ctx->max_cluster));
-  cudaError_t e = dbl ? launch_front<double>(a, ctx->max_ny, ctx->max_nx, st) : launch_front<float>(a, ctx->max_ny, ctx->max_nx, st);
-  CK(e, "local solve kernel");
+  a.cluster = clus;
+  CK(run_front(ctx, a, st), "local solve kernel");
   ctx->launches += 2;
   return check_kernel_err(ctx, st);
 }

@@ -375,7 +375,7 @@ void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const Fr
           flatten(kv.second, r, [&](const std::vector<std::pair<size_t, size_t>>&, int count) {
             ++n_items;
             maxs = std::max(maxs, count);
-            fac_elems += 2.0 * cl.nx * (double)cl.ny * cl.ldn;
+            fac_elems += 2.0 * cl.nx * (double)cl.blk;
           });
         }
         if (n_items == 0) continue;
@@ -431,7 +431,7 @@ void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const Fr
         }
         it.slot_count = count;
         const int rs = plan.tc_scratch ? std::max(front_rpad(count), front_tc_slots(count)) : front_rpad(count);
-        it.scratch_off = (long long)(cl.nx + 1) * rs * cl.ny;   // its size, for now
+        it.scratch_off = item_scratch(cl, rs, best_cl, plan.sym);   // its size, for now
         F.max_slots = std::max(F.max_slots, it.slot_count);
         items.push_back(it);
         F.item_count++;

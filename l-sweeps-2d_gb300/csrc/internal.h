@@ -50,12 +50,43 @@ struct DevCell {
   int I, J;
   int nx, ny;          // x-lines (block count) and points per line (block size)
   int lox, loy;        // global DOF of local (0, 0)
-  int ldn;             // leading dimension of a factor block (column-major)
-  int pad0;
+  int ldn;             // leading dimension of a whole factor block (column-major)
+  int blk;             // elements of a line's factor block: ny * ldn, or SymTiles::elems(ny)
   int lx[2][4], ly[2][4];
   int ownx[2][2], owny[2][2];
   long long fac_off;   // element offset of block 0 in the factor pool
-  long long prof_off;  // offset into the profile array: x-profiles (3*nx), then y (3*ny)
+  long long prof_off;  // offset into the profile array: x (lo, hi, dg: 3*nx), then y (lo, hi, dg, off, e: 5*ny)
+};
+
+// Factors in symmetric tiles (complex64, bf16 split; sweep_sym.cuh):
+// the lower half of each line's inverse E^-1 S^-1 E as 16 x 16 tiles, tile
+// (I, J), I >= J, in class (I + J) mod 4; the classes in turn, each ordered by
+// column, then row.  complex64: element (i, j) of a tile at 16 j + (i ^ swz(j));
+// split: planes of 8 x 8 bf16 matrices (sym_put in kernels_factor.cu).
+constexpr int kSymTilesMax = 12;   // tile rows: 192 points per line
+struct SymTiles {
+  static constexpr __host__ __device__ int rows(int ny) { return (ny + 15) >> 4; }
+  static constexpr __host__ __device__ int elems(int ny) { return rows(ny) * (rows(ny) + 1) / 2 * 256; }
+  static constexpr __host__ __device__ int swz(int j) { return ((j & 3) << 2) | (j >> 2); }
+};
+// per number of tile rows nb: the first tile of class q (first[nb][4]: the tile
+// count) and of class q's tiles in column j
+struct SymTable {
+  unsigned char first[kSymTilesMax + 1][8];
+  unsigned char column[kSymTilesMax + 1][4][kSymTilesMax];
+  constexpr SymTable() : first(), column() {
+    for (int nb = 0; nb <= kSymTilesMax; ++nb) {
+      int n = 0;
+      for (int q = 0; q < 4; ++q) {
+        first[nb][q] = (unsigned char)n;
+        for (int j = 0; j < kSymTilesMax; ++j) {
+          column[nb][q][j] = (unsigned char)n;
+          for (int i = j; i < nb; ++i) n += ((i + j) & 3) == q ? 1 : 0;
+        }
+      }
+      first[nb][4] = (unsigned char)n;
+    }
+  }
 };
 
 enum SlotKind : int {
@@ -146,6 +177,7 @@ struct FrontPlan {
   // items may run with tensor-core line products (8 or 16 slots, fewer
   // padded): their forward storage is sized for that many slots
   bool tc_scratch = false;
+  bool sym = false;          // factors in symmetric tiles
   // one launch per (step, sweep) instead of one per step (see kLanePlanes);
   // the cost model then counts a stage-2 / stage-3 launch as sharing the GPU
   // with `lane_concurrency` others of its size
@@ -206,11 +238,12 @@ struct FrontArgs {
   int* err;               // bit 1: a bounded wait timed out
   int cluster;            // CTAs per item (thread-block cluster size)
   int stages;             // shared-memory ring depth (set by the launcher)
-  int chunk;              // factor columns per streamed chunk (set by the launcher)
-  int ksw;                // consumer column slices (set by the launcher)
-  int split;              // factors hold bf16 hi/lo terms; the matvec runs on mma.sync
+  int chunk;              // factor columns per streamed chunk; symmetric tiles: bytes per ring stage (set by the launcher)
+  int ksw;                // consumer column slices; symmetric tiles: tile classes per chunk (set by the launcher)
+  int split;              // symmetric tiles hold bf16 hi/lo terms; the products run on mma.sync
   int tc;                 // complex64 line products on the tensor cores (tcgen05, 8 or 16 slots)
   long long wait_cycles;  // bounded-wait limit in clock cycles
+  const SymTable* symt;   // symmetric tiles: the tile order (device memory)
 };
 // CTAs per half of an item (the item's cluster holds two halves) for a
 // front of `items` cell solves on `nsm` SMs, with at most `max_cta` CTAs per item
@@ -221,23 +254,42 @@ inline int front_cluster(int items, int nsm, int max_cta) {
 }
 
 template <typename T> cudaError_t launch_front(const FrontArgs& a, int max_ny, int max_nx, cudaStream_t st);
+// the symmetric-tile kernel of a cluster size
+typedef void (*SymKernel)(FrontArgs);
+SymKernel sym_kernel_1(bool split);
+SymKernel sym_kernel_2(bool split);
+SymKernel sym_kernel_4(bool split);
+// the same front on factors in symmetric tiles (complex64, or bf16 split with a.split)
+cudaError_t launch_front_sym(const FrontArgs& a, int max_ny, int max_nx, cudaStream_t st);
 // clusters of `cluster` CTAs of the sweep-front kernel resident at once (one CTA per SM)
 int front_max_clusters(bool dbl, int cluster);
+int sym_max_clusters(bool split, int cluster);
 int front_rmax(bool dbl);
 int front_rpad(int n);
 // bit CL (1, 2, 4) set where items of `slots` slots on clusters of 2 CL CTAs fit in shared memory
-int front_fit_mask(bool dbl, bool split, int max_ny, int max_nx, int slots, bool tc = false);
+int front_fit_mask(bool dbl, int max_ny, int max_nx, int slots, bool tc = false);
+int sym_fit_mask(bool split, int max_ny, int max_nx, int slots);
+// scratch elements of an item on `cl` CTAs per half: y_k and x_k rows, shared
+// but for symmetric tiles on more than one CTA; an even number, so that the
+// items after it stay aligned for 16-byte accesses
+inline long long item_scratch(const DevCell& c, int slots_padded, int cl, bool sym) {
+  const long long n = (long long)(c.nx + 1) * slots_padded * c.ny * (sym && cl > 1 ? 2 : 1);
+  return (n + 1) & ~1LL;
+}
 // slots of a tensor-core item (8 or 16) for items of at most n slots
 int front_tc_slots(int n);
-// split: write every factor entry as bf16 hi/lo terms; `prev` then holds the
-// previous FP32 block of each cell's two half chains (2 x ny x ldn complex per
-// cell) for the Schur recurrences.  lookahead: factor each next panel while
+// Factor layouts: whole blocks, or symmetric tiles of FP32 values or of bf16
+// hi/lo terms.  With tiles `prev` holds the previous whole FP32 block of each
+// cell's two half chains (2 x ny x ldn complex per cell) for the Schur
+// recurrences, and the blocks are those of the symmetrised matrix.
+enum FactorLayout : int { FL_WHOLE = 0, FL_SYM = 1, FL_SYM_SPLIT = 2 };
+// lookahead: factor each next panel while
 // the current block's update runs on the other warps.
 template <typename T> cudaError_t launch_factorize(const DevCell* cells, int ncell, const double2* prof,
                                                    const double* mgrid, int n_dof, double omega2,
                                                    void* fac, void* prev, int max_ny, int* status,
-                                                   cudaStream_t st, bool split, bool lookahead,
-                                                   long long wait_cycles);
+                                                   cudaStream_t st, int layout, bool lookahead,
+                                                   long long wait_cycles, const SymTable* symt);
 // one bounded wait on a barrier that nothing completes (bit 1 of *err when it runs out)
 cudaError_t launch_wait_probe(int* err, long long limit_cycles, cudaStream_t st);
 size_t factor_smem_bytes(int ny, bool dbl);
@@ -247,7 +299,7 @@ size_t factor_smem_bytes(int ny, bool dbl);
 bool factorize_tc_supported(int max_ny);
 cudaError_t launch_factorize_tc(const DevCell* cells, int ncell, const double2* prof, const double* mgrid, int n_dof,
                                 double omega2, void* fac, void* prev, int max_ny, int* status, cudaStream_t st,
-                                bool split, long long wait_cycles);
+                                int layout, long long wait_cycles, const SymTable* symt);
 
 cudaError_t launch_apply_A(const double2* x, double2* y, int nrhs, int n_dof, const double2* gprof,
                            const double* mgrid, double omega2, cudaStream_t st);

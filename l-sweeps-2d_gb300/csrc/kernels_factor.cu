@@ -124,12 +124,30 @@ __device__ __forceinline__ void bf16_split(float x, unsigned& hi, unsigned& lo) 
   hi = (unsigned)__bfloat16_as_ushort(h);
   lo = (unsigned)__bfloat16_as_ushort(l);
 }
-// one factor entry of the split layout: {hi(re) | hi(im) << 16, lo(re) | lo(im) << 16}
-__device__ __forceinline__ uint2 split_entry(float2 v) {
-  unsigned hr, lr, hi_, li;
-  bf16_split(v.x, hr, lr);
-  bf16_split(v.y, hi_, li);
-  return make_uint2(hr | (hi_ << 16), lr | (li << 16));
+
+// Entry (i, j) of a line's factor into its symmetric tile (tab:
+// SymTable::column of the cell); complex64: the tiles of (i, j), i's tile row not
+// above j's; split: of (j, i), so that neighbouring threads (i) write
+// neighbouring values of a row.
+__device__ __forceinline__ void sym_put(float2* blk, const unsigned char* tab, int i, int j, float2 v, bool split) {
+  const int bi = i >> 4, bj = j >> 4;
+  if (split ? bi > bj : bi < bj) return;
+  const int hi = max(bi, bj), lo = min(bi, bj);
+  const int tile = tab[((bi + bj) & 3) * kSymTilesMax + lo] + ((hi - lo) >> 2);
+  if (!split) {
+    blk[tile * 256 + (j & 15) * 16 + ((i & 15) ^ SymTiles::swz(j & 15))] = v;
+    return;
+  }
+  // planes re hi, im hi, re lo, im lo of four 8 x 8 blocks (by column, then row) of bf16, row j mod 16, column i mod 16
+  unsigned short* p = reinterpret_cast<unsigned short*>(blk) + tile * 1024 +
+                      (((j >> 3) & 1) + ((i >> 3) & 1) * 2) * 64 + (j & 7) * 8 + (i & 7);
+  unsigned h, l;
+  bf16_split(v.x, h, l);
+  p[0] = (unsigned short)h;
+  p[512] = (unsigned short)l;
+  bf16_split(v.y, h, l);
+  p[256] = (unsigned short)h;
+  p[768] = (unsigned short)l;
 }
 
 // block-column owner: CTA g owns the columns [g n/G, (g+1) n/G)
@@ -206,8 +224,8 @@ template <typename T>
 __global__ void __launch_bounds__(kFT, 1)
 k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
             const double* __restrict__ mgrid, int n_dof, double omega2, cx_t<T>* __restrict__ fac,
-            cx_t<T>* __restrict__ prev, long long prev_stride, int split, int middle, int lookahead, int G,
-            int nmax, int ldw, int* status, long long wait_cycles) {
+            cx_t<T>* __restrict__ prev, long long prev_stride, int layout, int middle, int lookahead, int G,
+            int nmax, int ldw, int* status, long long wait_cycles, const SymTable* __restrict__ symt) {
   using C = cx_t<T>;
   constexpr int CJ = FacCfg<T>::CJ;
   constexpr int kB = FacCfg<T>::B;
@@ -233,6 +251,9 @@ k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 8);
   unsigned* wkey = reinterpret_cast<unsigned*>(smem + 16);    // [2][8] per-warp pivot keys by step parity
   uint64_t* exitbar = reinterpret_cast<uint64_t*>(smem + 128); // every CTA of the cluster is done
+  unsigned char* tab = smem + 144;                            // [4][kSymTilesMax] symmetric tiles: first tile per column
+  static_assert(144 + 4 * kSymTilesMax <= 256, "header");
+  const bool sym = layout != FL_WHOLE;
   int* used = reinterpret_cast<int*>(smem + 256);             // [nmax]
   int* piv = used + kMaxN;                                     // [nmax]
   int* pslot = piv + kMaxN;                                    // [nmax] block pivot slot of a row, -1 if none
@@ -244,10 +265,13 @@ k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
   C* W = U + kB * ldw;                                         // [nmax][ldw], my columns
   C* RowB = W + (size_t)nmax * ldw;                            // [2][kB][kMaxN] panel rows by step parity
 
-  const double2* px = prof + cl.prof_off;  // lo_x, hi_x, dg_x, lo_y, hi_y, dg_y
+  const double2* px = prof + cl.prof_off;  // lo_x, hi_x, dg_x, lo_y, hi_y, dg_y, off_y, e_y
   const double2* py = px + 3 * nx;
+  // couplings of row i to i - 1 and i + 1: those of the symmetrised matrix for symmetric tiles
+  const double2* cs = sym ? py + 3 * n : py;
+  const double2* cn = sym ? py + 3 * n + 1 : py + n;
   C* Fac = fac + cl.fac_off;
-  // split: the last inverse of each half chain in FP32, [cell][half]
+  // symmetric tiles: the last whole inverse of each half chain, [cell][half]
   C* Prev0 = prev ? prev + (long long)(2 * cidx) * prev_stride : nullptr;
   C* Prev1 = prev ? Prev0 + prev_stride : nullptr;
   C* Prev = half ? Prev1 : Prev0;
@@ -260,6 +284,8 @@ k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < kMaxN; i += kFT) pslot[i] = -1;
+  if (sym && tid < 4 * kSymTilesMax)
+    tab[tid] = symt->column[SymTiles::rows(n)][tid / kSymTilesMax][tid % kSymTilesMax];
   __syncthreads();
   if (G > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 
@@ -317,13 +343,13 @@ k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
     if (middle) {
       coupa = cmul(to_c(px[k], z), to_c(px[nx + k - 1], z));   // w_m e_{m-1}
       coupb = cmul(to_c(px[nx + k], z), to_c(px[k + 1], z));   // e_m w_{m+1}
-      Fa = split ? Prev0 : Fac + (size_t)(k - 1) * n * ldn;
-      Fb = split ? Prev1 : Fac + (size_t)(k + 1) * n * ldn;
+      Fa = sym ? Prev0 : Fac + (size_t)(k - 1) * cl.blk;
+      Fb = sym ? Prev1 : Fac + (size_t)(k + 1) * cl.blk;
     } else if (step > 0) {
       const int kp = half == 0 ? k - 1 : k + 1;
       coupa = half == 0 ? cmul(to_c(px[k], z), to_c(px[nx + k - 1], z))    // w_k e_{k-1}
                         : cmul(to_c(px[nx + k], z), to_c(px[k + 1], z));   // e_k w_{k+1}
-      Fa = split ? Prev : Fac + (size_t)kp * n * ldn;
+      Fa = sym ? Prev : Fac + (size_t)kp * cl.blk;
     }
     const double* mrow = mgrid + (long long)(cl.lox + k) * n_dof + cl.loy;
     for (int e = tid; e < n * nc; e += kFT) {
@@ -336,9 +362,9 @@ k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
         d.x -= (T)(omega2 * mrow[i]);
         v = cadd(v, d);
       } else if (j == i - 1) {
-        v = cadd(v, to_c(py[i], z));          // coupling to j-1 (south)
+        v = cadd(v, to_c(cs[i], z));          // coupling to j-1 (south)
       } else if (j == i + 1) {
-        v = cadd(v, to_c(py[n + i], z));      // coupling to j+1 (north)
+        v = cadd(v, to_c(cn[i], z));          // coupling to j+1 (north)
       }
       W[(size_t)i * ldw + cc] = v;
     }
@@ -545,19 +571,25 @@ k_factorize(const DevCell* __restrict__ cells, const double2* __restrict__ prof,
     }
 
     // ---- unscramble my columns: output column piv[c] holds W[piv[i]][c] ----
-    C* Fk = Fac + (size_t)k * n * ldn;
-    for (int e = tid; e < nc * ldn; e += kFT) {
-      const int cc = e / ldn, i = e - cc * ldn;
+    C* Fk = Fac + (size_t)k * cl.blk;
+    const int rows = sym ? 16 * SymTiles::rows(n) : ldn;   // zeros past n
+    for (int e = tid; e < nc * rows; e += kFT) {
+      const int cc = e / rows, i = e - cc * rows;
       const int j = piv[c0 + cc];
       const C v = (i < n) ? W[(size_t)piv[i] * ldw + cc] : z;
       if constexpr (sizeof(T) == 4) {
-        if (split) {
-          if (!middle) Prev[(size_t)j * ldn + i] = v;
-          reinterpret_cast<uint2*>(Fk)[(size_t)j * ldn + i] = split_entry(v);
+        if (sym) {
+          if (!middle && i < n) Prev[(size_t)j * ldn + i] = v;
+          sym_put(Fk, tab, i, j, v, layout == FL_SYM_SPLIT);
           continue;
         }
       }
       Fk[(size_t)j * ldn + i] = v;
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (sym && (int)g == G - 1)   // the columns past n
+        for (int e = tid; e < (rows - n) * rows; e += kFT)
+        sym_put(Fk, tab, e % rows, n + e / rows, z, layout == FL_SYM_SPLIT);
     }
     // the next line's Schur complement reads every CTA's columns of Sinv_k
     if (!csync()) { leave(); return; }
@@ -602,7 +634,8 @@ size_t factor_smem_bytes(int ny, bool dbl) {
 template <typename T>
 cudaError_t launch_factorize(const DevCell* cells, int ncell, const double2* prof, const double* mgrid,
                              int n_dof, double omega2, void* fac, void* prev, int max_ny, int* status,
-                             cudaStream_t st, bool split, bool lookahead, long long wait_cycles) {
+                             cudaStream_t st, int layout, bool lookahead, long long wait_cycles,
+                             const SymTable* symt) {
   if (ncell <= 0) return cudaSuccess;
   if (max_ny > kMaxN) return cudaErrorInvalidValue;
   int dev = 0, maxopt = 0, ldw = 0;
@@ -616,8 +649,8 @@ cudaError_t launch_factorize(const DevCell* cells, int ncell, const double2* pro
   // host threads launching concurrently never lower it under one another
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt);
   if (e != cudaSuccess) return e;
-  if (split && (sizeof(T) != 4 || prev == nullptr)) return cudaErrorInvalidValue;
-  // split: the last FP32 inverse of each half chain, max_ny x ldn_max complex
+  if (layout != FL_WHOLE && (sizeof(T) != 4 || prev == nullptr || symt == nullptr)) return cudaErrorInvalidValue;
+  // symmetric tiles: the last whole FP32 inverse of each half chain, max_ny x ldn_max complex
   // per (cell, half) (ldn_max <= max_ny + 7)
   const long long prev_stride = (long long)max_ny * (max_ny + 8);
   cudaLaunchConfig_t cfg{};
@@ -635,8 +668,8 @@ cudaError_t launch_factorize(const DevCell* cells, int ncell, const double2* pro
   for (int middle = 0; middle < 2; ++middle) {
     cfg.gridDim = dim3((unsigned)(ncell * G * (middle ? 1 : 2)));
     e = cudaLaunchKernelEx(&cfg, kern, cells, prof, mgrid, n_dof, omega2, reinterpret_cast<cx_t<T>*>(fac),
-                           reinterpret_cast<cx_t<T>*>(split ? prev : nullptr), prev_stride, split ? 1 : 0, middle,
-                           lookahead ? 1 : 0, G, max_ny, ldw, status, wait_cycles);
+                           reinterpret_cast<cx_t<T>*>(layout != FL_WHOLE ? prev : nullptr), prev_stride, layout, middle,
+                           lookahead ? 1 : 0, G, max_ny, ldw, status, wait_cycles, symt);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -644,8 +677,8 @@ cudaError_t launch_factorize(const DevCell* cells, int ncell, const double2* pro
 
 
 template cudaError_t launch_factorize<float>(const DevCell*, int, const double2*, const double*, int, double,
-                                             void*, void*, int, int*, cudaStream_t, bool, bool, long long);
+                                             void*, void*, int, int*, cudaStream_t, int, bool, long long, const SymTable*);
 template cudaError_t launch_factorize<double>(const DevCell*, int, const double2*, const double*, int, double,
-                                              void*, void*, int, int*, cudaStream_t, bool, bool, long long);
+                                              void*, void*, int, int*, cudaStream_t, int, bool, long long, const SymTable*);
 
 }  // namespace lsw

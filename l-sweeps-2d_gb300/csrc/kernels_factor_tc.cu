@@ -80,7 +80,8 @@ constexpr int kOffPb = kOffInts + 4 * kMaxRows * 4;                // int [2][kB
 constexpr int kOffKey = kOffPb + 2 * kB * 4;                       // unsigned [2][8]
 constexpr int kOffBar = kOffKey + 64;                              // 3 mbarriers
 constexpr int kOffMisc = kOffBar + 24;                             // abort flag, TMEM address
-constexpr int kSmem = kOffMisc + 16;
+constexpr int kOffTab = kOffMisc + 16;                             // unsigned char [4][kSymTilesMax]
+constexpr int kSmem = kOffTab + 4 * kSymTilesMax;
 static_assert(kOffF == 86016, "layout");
 static_assert(16 * kMaxRows * 8 <= 3 * kATerm, "unscramble staging tile [16][ldn] fits in the A operand area");
 static_assert(kOffBar % 8 == 0, "mbarrier alignment");
@@ -233,11 +234,30 @@ __device__ __forceinline__ void bf16_split(float x, unsigned& hi, unsigned& lo) 
   hi = (unsigned)__bfloat16_as_ushort(h);
   lo = (unsigned)__bfloat16_as_ushort(l);
 }
-__device__ __forceinline__ uint2 split_entry(float2 v) {
-  unsigned hr, lr, hi_, li;
-  bf16_split(v.x, hr, lr);
-  bf16_split(v.y, hi_, li);
-  return make_uint2(hr | (hi_ << 16), lr | (li << 16));
+
+// Entry (i, j) of a line's factor into its symmetric tile (tab:
+// SymTable::column of the cell); complex64: the tiles of (i, j), i's tile row not
+// above j's; split: of (j, i), so that neighbouring threads (i) write
+// neighbouring values of a row.
+__device__ __forceinline__ void sym_put(float2* blk, const unsigned char* tab, int i, int j, float2 v, bool split) {
+  const int bi = i >> 4, bj = j >> 4;
+  if (split ? bi > bj : bi < bj) return;
+  const int hi = max(bi, bj), lo = min(bi, bj);
+  const int tile = tab[((bi + bj) & 3) * kSymTilesMax + lo] + ((hi - lo) >> 2);
+  if (!split) {
+    blk[tile * 256 + (j & 15) * 16 + ((i & 15) ^ SymTiles::swz(j & 15))] = v;
+    return;
+  }
+  // planes re hi, im hi, re lo, im lo of four 8 x 8 blocks (by column, then row) of bf16, row j mod 16, column i mod 16
+  unsigned short* p = reinterpret_cast<unsigned short*>(blk) + tile * 1024 +
+                      (((j >> 3) & 1) + ((i >> 3) & 1) * 2) * 64 + (j & 7) * 8 + (i & 7);
+  unsigned h, l;
+  bf16_split(v.x, h, l);
+  p[0] = (unsigned short)h;
+  p[512] = (unsigned short)l;
+  bf16_split(v.y, h, l);
+  p[256] = (unsigned short)h;
+  p[768] = (unsigned short)l;
 }
 
 __device__ __forceinline__ int col_owner(int j, int n, int G) { return ((j + 1) * G - 1) / n; }
@@ -245,7 +265,8 @@ __device__ __forceinline__ int col_owner(int j, int n, int G) { return ((j + 1) 
 __global__ void __launch_bounds__(kT, 1)
 k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ prof, const double* __restrict__ mgrid,
                int n_dof, double omega2, float2* __restrict__ fac, float2* __restrict__ prev, long long prev_stride,
-               int split, int middle, int G, int* status, long long wait_cycles) {
+               int layout, int middle, int G, int* status, long long wait_cycles,
+               const SymTable* __restrict__ symt) {
   using C = float2;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -287,8 +308,14 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kOffMisc);
   unsigned* tslot = reinterpret_cast<unsigned*>(smem + kOffMisc + 4);
 
-  const double2* px = prof + cl.prof_off;  // lo_x, hi_x, dg_x, lo_y, hi_y, dg_y
+  unsigned char* tab = smem + kOffTab;
+  const bool sym = layout != FL_WHOLE;
+
+  const double2* px = prof + cl.prof_off;  // lo_x, hi_x, dg_x, lo_y, hi_y, dg_y, off_y, e_y
   const double2* py = px + 3 * nx;
+  // couplings of row i to i - 1 and i + 1: those of the symmetrised matrix for symmetric tiles
+  const double2* cs = sym ? py + 3 * n : py;
+  const double2* cn = sym ? py + 3 * n + 1 : py + n;
   C* Fac = fac + cl.fac_off;
   C* Prev0 = prev ? prev + (long long)(2 * cidx) * prev_stride : nullptr;
   C* Prev1 = prev ? Prev0 + prev_stride : nullptr;
@@ -309,6 +336,8 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < kMaxRows; i += kT) pslot[i] = -1;
+  if (sym && tid < 4 * kSymTilesMax)
+    tab[tid] = symt->column[SymTiles::rows(n)][tid / kSymTilesMax][tid % kSymTilesMax];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -404,13 +433,13 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
     if (middle) {
       coupa = cmul(to_c(px[k], z), to_c(px[nx + k - 1], z));   // w_m e_{m-1}
       coupb = cmul(to_c(px[nx + k], z), to_c(px[k + 1], z));   // e_m w_{m+1}
-      Fa = split ? Prev0 : Fac + (size_t)(k - 1) * n * ldn;
-      Fb = split ? Prev1 : Fac + (size_t)(k + 1) * n * ldn;
+      Fa = sym ? Prev0 : Fac + (size_t)(k - 1) * cl.blk;
+      Fb = sym ? Prev1 : Fac + (size_t)(k + 1) * cl.blk;
     } else if (step > 0) {
       const int kp = half == 0 ? k - 1 : k + 1;
       coupa = half == 0 ? cmul(to_c(px[k], z), to_c(px[nx + k - 1], z))    // w_k e_{k-1}
                         : cmul(to_c(px[nx + k], z), to_c(px[k + 1], z));   // e_k w_{k+1}
-      Fa = split ? Prev : Fac + (size_t)kp * n * ldn;
+      Fa = sym ? Prev : Fac + (size_t)kp * cl.blk;
     }
     if (warp_rows) {
       C dr = z, lo = z, hi = z;
@@ -418,8 +447,8 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
         const double* mrow = mgrid + (long long)(cl.lox + k) * n_dof + cl.loy;
         dr = cadd(dgx, to_c(py[2 * n + r], z));
         dr.x -= (float)(omega2 * mrow[r]);
-        lo = to_c(py[r], z);        // coupling to j = r - 1 (south)
-        hi = to_c(py[n + r], z);    // coupling to j = r + 1 (north)
+        lo = to_c(cs[r], z);   // coupling to j = r - 1 (south)
+        hi = to_c(cn[r], z);   // coupling to j = r + 1 (north)
       }
       for (int cb = 0; cb < nc; cb += 16) {
         float v[32];
@@ -722,7 +751,8 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
     for (int i = tid; i < n; i += kT) pinv[piv[i]] = i;
     __syncthreads();
     C* stg = reinterpret_cast<C*>(smem + kOffA);     // [16][ldn]
-    C* Fk = Fac + (size_t)k * n * ldn;
+    C* Fk = Fac + (size_t)k * cl.blk;
+    const int rows = sym ? 16 * SymTiles::rows(n) : ldn;   // zeros past n
     for (int cb = 0; cb < nc; cb += 16) {
       if (warp_rows) {
         float v[32];
@@ -736,19 +766,22 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
       }
       __syncthreads();
       const int ncol = min(16, nc - cb);
-      for (int e = tid; e < ncol * ldn; e += kT) {
-        const int q = e / ldn, i = e - q * ldn;
+      for (int e = tid; e < ncol * rows; e += kT) {
+        const int q = e / rows, i = e - q * rows;
         const int j = piv[c0 + cb + q];
         const C val = i < n ? stg[(size_t)q * ldn + i] : z;
-        if (split) {
-          if (!middle) Prev[(size_t)j * ldn + i] = val;
-          reinterpret_cast<uint2*>(Fk)[(size_t)j * ldn + i] = split_entry(val);
+        if (sym) {
+          if (!middle && i < n) Prev[(size_t)j * ldn + i] = val;
+          sym_put(Fk, tab, i, j, val, layout == FL_SYM_SPLIT);
         } else {
           Fk[(size_t)j * ldn + i] = val;
         }
       }
       __syncthreads();
     }
+    if (sym && (int)g == G - 1)   // the columns past n
+      for (int e = tid; e < (rows - n) * rows; e += kT)
+        sym_put(Fk, tab, e % rows, n + e / rows, z, layout == FL_SYM_SPLIT);
     // the next line's Schur complement reads every CTA's columns of this inverse
     if (!csync()) { leave(); return; }
   }
@@ -763,11 +796,11 @@ bool factorize_tc_supported(int max_ny) { return max_ny >= 1 && max_ny <= kMaxRo
 
 cudaError_t launch_factorize_tc(const DevCell* cells, int ncell, const double2* prof, const double* mgrid, int n_dof,
                                 double omega2, void* fac, void* prev, int max_ny, int* status, cudaStream_t st,
-                                bool split, long long wait_cycles) {
+                                int layout, long long wait_cycles, const SymTable* symt) {
   if (ncell <= 0) return cudaSuccess;
   const int G = tc_cluster(max_ny);
   if (G == 0) return cudaErrorInvalidValue;
-  if (split && prev == nullptr) return cudaErrorInvalidValue;
+  if (layout != FL_WHOLE && (prev == nullptr || symt == nullptr)) return cudaErrorInvalidValue;
   int dev = 0, maxopt = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -789,8 +822,8 @@ cudaError_t launch_factorize_tc(const DevCell* cells, int ncell, const double2* 
   for (int middle = 0; middle < 2; ++middle) {
     cfg.gridDim = dim3((unsigned)(ncell * G * (middle ? 1 : 2)));
     e = cudaLaunchKernelEx(&cfg, k_factorize_tc, cells, prof, mgrid, n_dof, omega2, reinterpret_cast<float2*>(fac),
-                           reinterpret_cast<float2*>(split ? prev : nullptr), prev_stride, split ? 1 : 0, middle, G,
-                           status, wait_cycles);
+                           reinterpret_cast<float2*>(layout != FL_WHOLE ? prev : nullptr), prev_stride, layout, middle, G,
+                           status, wait_cycles, symt);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

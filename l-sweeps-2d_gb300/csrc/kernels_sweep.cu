@@ -1,5 +1,7 @@
-// Sweep-front kernel: every cell solve of one front of the L-sweep
-// preconditioner in one launch.
+// Sweep-front kernel for whole factor blocks (complex128, and complex64 of
+// contexts that run tensor-core line products): every cell solve of one front of
+// the L-sweep preconditioner in one launch.  complex64 and bf16-split factors
+// otherwise come in symmetric tiles (sweep_sym.cuh).
 //
 // A cell matrix is block tridiagonal over its x-lines (DOF order i*ny + j,
 // AssemblerHelmholtz2DFD.cpp:166-177); the couplings between lines are scalar
@@ -40,11 +42,8 @@
 // warp 3 copies y_k (forward) and x_k (backward) to a per-item scratch; the
 // remaining warps are consumers: a lane owns a row pair of a 64-row group and
 // a warp one of KSW interleaved column slices, accumulating in registers with
-// no cross-lane reduction (complex FP32/FP64 FMAs).  With split factors (bf16
-// hi + lo words) a consumer warp owns a 16-row m-tile instead and runs the
-// partial products on the tensor cores (mma.sync m16n8k16, three products per
-// k-step, FP32 accumulation) against the line input staged as bf16 hi/lo
-// words.  Line vectors and partial sums are stored [column][slot] so that
+// no cross-lane reduction (complex FP32/FP64 FMAs).
+// Line vectors and partial sums are stored [column][slot] so that
 // slot offsets are compile-time constants.  The
 // outputs (owned DOFs, trace lines, cell vectors) are written once per item
 // from the scratch by every non-producer thread after the backward pass, each
@@ -63,8 +62,7 @@
 // DDCheckerboard.cpp:744-772) and its outgoing trace lines into the trace pool.
 #include "common.cuh"
 #include "internal.h"
-
-#include <cuda_bf16.h>
+#include "sweep_common.cuh"
 
 #include <algorithm>
 
@@ -78,137 +76,6 @@ constexpr int kAux = 4;               // producer, two helper warps, writer warp
 constexpr int kNSMax = 8;             // ring stages
 constexpr int kHdr = 256;             // barrier header bytes
 constexpr int SK_NONE = 99;           // padding slot
-constexpr unsigned kSuspendNs = 1000000;          // try_wait sleeps up to 1 ms (woken by the phase)
-
-
-// ---------------------------------------------------------------------------
-// PTX helpers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned saddr(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned cluster_size() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ unsigned mapa(unsigned a, unsigned rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_init(uint64_t* b, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
-}
-// arrive on the barrier at the same offset in CTA `rank` of the cluster (release, cluster scope)
-__device__ __forceinline__ void mbar_arrive_remote(uint64_t* b, unsigned rank) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(saddr(b), rank))
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(saddr(b)), "r"(parity), "r"(kSuspendNs)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(saddr(b)), "r"(parity), "r"(kSuspendNs)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait (see the file comment): gives up after `limit` clock cycles,
-// or at once when the CTA's abort flag is up (abort_flag == nullptr: a wait
-// that only the limit ends, for the drain before leaving).
-template <bool CLUSTER>
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity, int* err, volatile int* abort_flag,
-                                          long long limit) {
-  auto tw = [&]() { return CLUSTER ? mbar_try_wait_cluster(b, parity) : mbar_try_wait(b, parity); };
-  if (tw()) return true;
-  const long long t0 = clock64();
-  while (true) {
-    if (abort_flag && *abort_flag) return false;
-    if (tw()) return true;
-    if (clock64() - t0 > limit) {
-      if (abort_flag) *abort_flag = 1;
-      atomicOr(err, 2);
-      return false;
-    }
-  }
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   saddr(dst)),
-               "l"(src), "r"(bytes), "r"(saddr(bar))
-               : "memory");
-}
-__device__ __forceinline__ void named_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-// store into CTA `rank`'s shared memory; the bytes complete the transaction
-// count of that CTA's mbarrier at the same offset as `bar`
-__device__ __forceinline__ void st_async(float2* p, unsigned rank, float2 v, uint64_t* bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(
-                   mapa(saddr(p), rank)),
-               "f"(v.x), "f"(v.y), "r"(mapa(saddr(bar), rank))
-               : "memory");
-}
-__device__ __forceinline__ void st_async2(float2* p, unsigned rank, float2 v0, float2 v1, uint64_t* bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
-                   mapa(saddr(p), rank)),
-               "f"(v0.x), "f"(v0.y), "f"(v1.x), "f"(v1.y), "r"(mapa(saddr(bar), rank))
-               : "memory");
-}
-__device__ __forceinline__ void st_async(double2* p, unsigned rank, double2 v, uint64_t* bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
-                   mapa(saddr(p), rank)),
-               "d"(v.x), "d"(v.y), "r"(mapa(saddr(bar), rank))
-               : "memory");
-}
-__device__ __forceinline__ void red_add(float2* p, float2 v) {
-  atomicAdd(&p->x, v.x);
-  atomicAdd(&p->y, v.y);
-}
-__device__ __forceinline__ void red_add(double2* p, double2 v) {
-  atomicAdd(&p->x, v.x);
-  atomicAdd(&p->y, v.y);
-}
-
-// bf16x2 words of the hi and lo terms of (a, b): low half a, high half b
-__device__ __forceinline__ void split_pair(float a, float b, unsigned& hi, unsigned& lo) {
-  const __nv_bfloat16 ah = __float2bfloat16_rn(a), bh = __float2bfloat16_rn(b);
-  const __nv_bfloat16 al = __float2bfloat16_rn(a - __bfloat162float(ah));
-  const __nv_bfloat16 bl = __float2bfloat16_rn(b - __bfloat162float(bh));
-  hi = (unsigned)__bfloat16_as_ushort(ah) | ((unsigned)__bfloat16_as_ushort(bh) << 16);
-  lo = (unsigned)__bfloat16_as_ushort(al) | ((unsigned)__bfloat16_as_ushort(bl) << 16);
-}
-// D += A B, m16n8k16, bf16 operands, FP32 accumulation
-__device__ __forceinline__ void mma_bf16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
-                                         unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-               "{%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // ---- tensor-core (tcgen05) line products of complex64 items ----
 // A line's partial products D[row][n] = sum_k A[row][k] B[n][k] as real
 // GEMMs: A = the factor block with k = 2 column + (0: Re, 1: Im), B = the line
@@ -288,72 +155,6 @@ __device__ __forceinline__ void tm_ld(unsigned taddr, float (&v)[N]) {
 // CTA c of a cluster of CL owns rows/columns [c*ny/CL, (c+1)*ny/CL)
 __device__ __forceinline__ int owner_of(int row, int ny, int CL) { return ((row + 1) * CL - 1) / ny; }
 
-__device__ __forceinline__ bool is_line(int gnode, int m, int N) {
-  // interface lines k_b(J), k_b(J)+1 for J = 0..N-2 (the trace1/traceN rows
-  // zeroed by getSeparatedRHS)
-  if (gnode < m || gnode > (m + 1) * (N - 1)) return false;
-  const int r = gnode % (m + 1);
-  return r == m || r == 0;
-}
-
-struct SlotCoef {
-  double2 c_oi_x, c_io_x, c_oi_y, c_io_y;
-};
-
-template <typename T>
-__device__ __forceinline__ cx_t<T> rhs_elem(const FrontArgs& a, const DevCell& cl, const DevSlot& s,
-                                            const SlotCoef& cf, const cx_t<T>* tr, int k, int j) {
-  using C = cx_t<T>;
-  C z = czero<C>();
-  switch (s.kind) {
-    case SK_CELLVEC: {
-      const double2 v = a.x_in[(long long)s.rhs * a.x_stride + (long long)k * cl.ny + j];
-      return to_c(v, z);
-    }
-    case SK_DIR_X: {
-      if (k == s.xo) return cmul(to_c(cf.c_oi_x, z), tr[s.in_lr1 + j]);
-      if (k == s.xi) return cneg(cmul(to_c(cf.c_io_x, z), tr[s.in_lr0 + j]));
-      return z;
-    }
-    case SK_DIR_Y: {
-      if (j == s.yo) return cmul(to_c(cf.c_oi_y, z), tr[s.in_ud1 + k]);
-      if (j == s.yi) return cneg(cmul(to_c(cf.c_io_y, z), tr[s.in_ud0 + k]));
-      return z;
-    }
-    case SK_CORNER: {
-      // L-shaped sources: trace0 set L0 = {(xo, y): y inside yo} u {(x, yo): x inside xo},
-      // trace1 set L1 likewise on (xi, yi) (computeLTraceIndexSets, 1119-1277);
-      // rhs[L0] = A01 v1, rhs[L1] = -A10 v0 with the trace values of extractLTraces
-      // (UD0 > LR0 > UD1 > LR1 where lines cross).
-      const bool yin_o = (j - s.yo) * s.dy > 0;
-      const bool yin_i = (j - s.yi) * s.dy > 0;
-      if (k == s.xo) {
-        if (!yin_o) return z;
-        const C v = (j == s.yi) ? tr[s.in_ud1 + s.xi] : tr[s.in_lr1 + j];
-        return cmul(to_c(cf.c_oi_x, z), v);
-      }
-      const bool xin_i = (k - s.xi) * s.dx > 0;
-      if (k == s.xi) {
-        if (j == s.yo) return cmul(to_c(cf.c_oi_y, z), tr[s.in_ud1 + k]);
-        if (j == s.yi) {
-          C r = cneg(cmul(to_c(cf.c_io_x, z), tr[s.in_lr0 + j]));
-          cfms(r, to_c(cf.c_io_y, z), tr[s.in_ud0 + k]);
-          return r;
-        }
-        if (yin_i) return cneg(cmul(to_c(cf.c_io_x, z), tr[s.in_lr0 + j]));
-        return z;
-      }
-      if (xin_i) {
-        if (j == s.yo) return cmul(to_c(cf.c_oi_y, z), tr[s.in_ud1 + k]);
-        if (j == s.yi) return cneg(cmul(to_c(cf.c_io_y, z), tr[s.in_ud0 + k]));
-      }
-      return z;
-    }
-    default:
-      return z;
-  }
-}
-
 // two consecutive rows of one factor column, from shared memory
 template <typename T> struct Pair;
 template <> struct Pair<float> {
@@ -368,11 +169,11 @@ template <> struct Pair<double> {
   __device__ __forceinline__ void load(const double2* p) { a = p[0]; b = p[1]; }
 };
 
-template <typename T, int R, bool SPLIT, bool TCM = false>
+template <typename T, int R, bool TCM = false>
 __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it, const DevCell& cl, unsigned char* smem) {
   using C = cx_t<T>;
   // complex64 line products on the tensor cores (tcgen05, TMEM accumulators)
-  constexpr bool TC = TCM && !SPLIT && sizeof(T) == 4;
+  constexpr bool TC = TCM && sizeof(T) == 4;
   static_assert(!TC || R == 8 || R == 16, "tensor-core items carry 8 or 16 slots");
   constexpr int TN = 2 * R;                                  // GEMM n: (slot, Re / Im)
   constexpr int kTcCols = TN * 2 < 32 ? 32 : TN * 2;         // TMEM columns: two 128-row tiles
@@ -409,15 +210,13 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   const int jb = (int)crank * ny / CL, je = ((int)crank + 1) * ny / CL;
   const int nJ = je - jb;               // my columns / rows of every line
   const int RG = (ny + 63) >> 6;        // row groups of 64 rows
-  // consumer warps: KSW column slices per row group, or (split) one per 16-row m-tile
+  // consumer warps: KSW column slices per row group
   // FP32/FP64 FMA matvec: KSW column slices per row group; with more than 8
   // slots (complex64) two slot groups of R / 2 slots each, on their own warps,
   // so that a warp keeps at most 8 slots of two rows in registers
-  constexpr int SG = (!SPLIT && sizeof(T) == 4 && R > 8) ? 2 : 1;
+  constexpr int SG = (sizeof(T) == 4 && R > 8) ? 2 : 1;
   constexpr int RS = R / SG;
-  const int NCW = TC ? kMaxRG * kMaxKSW : SPLIT ? (ny + 15) >> 4 : KSW * RG * SG;
-  constexpr int NT = (2 * R + 7) / 8;   // split: n-tiles of 8 (Re, Im interleaved per slot)
-  constexpr int NT8 = NT * 8;
+  const int NCW = TC ? kMaxRG * kMaxKSW : KSW * RG * SG;
   const int NCT = NCW * 32;
   const int NSYNC = NCT + 96;           // consumers + 2 helper warps + writer warp
   const int nch = (nJ + CW - 1) / CW;   // chunks per line
@@ -468,7 +267,7 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   const size_t qbuf = (size_t)CL * qplane;
   p = al16(p + 2 * qbuf * sizeof(C));
   C* LS = reinterpret_cast<C*>(p);      // [KSW][R][64 RG] the column slices' partial sums, before their sum
-  if (!SPLIT && !TC) p = al16(p + (size_t)KSW * 64 * RG * R * sizeof(C));
+  if (!TC) p = al16(p + (size_t)KSW * 64 * RG * R * sizeof(C));
   // tensor-core items: the A stages ([stage][term][tile] 128 x 16 bf16) and the
   // line input as B ([term] TN x Kp bf16, Kp = my columns x 2 rounded to 32)
   const int MT = (ldn + 127) >> 7;
@@ -483,12 +282,6 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
     Bop = p;
     p = al16(p + (size_t)3 * b_term);
   }
-  // split: the next line's input as mma B words, hi and lo terms, [column][n]
-  // with n = 2 slot + (0: real part, 1: imaginary part) of the product
-  const int nJ8 = ((nJcap + 7) & ~7) + 8;
-  unsigned* BwH = reinterpret_cast<unsigned*>(p);
-  unsigned* BwL = BwH + (size_t)nJ8 * NT8;
-  if (SPLIT) p = al16(p + 2 * (size_t)nJ8 * NT8 * sizeof(unsigned));
   int* rowinfo = reinterpret_cast<int*>(p);   // [ny] owner CTA << 16 | row offset in the owner's range
   p = al16(p + sizeof(int) * ny);
   DevSlot* sl = reinterpret_cast<DevSlot*>(p);
@@ -544,13 +337,6 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   for (int k = tid; k < nx; k += blockDim.x) {
     wsh[k] = to_c(px[k], czero<C>());
     esh[k] = to_c(px[nx + k], czero<C>());
-  }
-  if constexpr (SPLIT) {
-    // the mma k-steps of a chunk's last columns and rows past ldn read ring
-    // entries no copy wrote; zeros (with zero B words past my columns) keep
-    // them finite and without effect
-    for (size_t i = tid; i < (size_t)NS * slot_elems; i += blockDim.x) ring[i] = czero<C>();
-    for (size_t i = tid; i < 2 * (size_t)nJ8 * NT8; i += blockDim.x) BwH[i] = 0u;
   }
   if constexpr (TC) {
     // A rows past ldn and B columns past my columns are never written: zeros
@@ -680,7 +466,7 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
       long long idx = 0;
       bool stopped = false;
       for (int li = 0; li < nline && !stopped; ++li) {
-        const C* blk = fac + (size_t)line_k(li) * ny * ldn;
+        const C* blk = fac + (size_t)line_k(li) * cl.blk;
         for (int c = 0; c < nch; ++c, ++idx) {
           if ((idx & 1) != lane) continue;   // lanes 0 and 1 issue alternate chunks
           const int slot = (int)(idx % NS);
@@ -773,24 +559,13 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   const int r0 = rg * 64 + 2 * lane;    // my row pair
   const bool rows_ok = r0 < ldn;
 
-  // split: the mma B words of input entry e = (column, slot) of the next line,
-  // n = 2 slot: (re, -im), n = 2 slot + 1: (im, re), hi and lo terms
+  // tensor-core items: entry e = (column, slot) of the next line's input as B
   auto write_bw = [&](int e, C v) {
     if constexpr (TC) {
       // B rows n = 2 slot (Re of the product): [Re, -Im]; n = 2 slot + 1: [Im, Re]
       const int jj = e / R, r = e - jj * R;
       put3(Bop, b_term, b_off(2 * r, 2 * jj, TN), v.x, -v.y);
       put3(Bop, b_term, b_off(2 * r + 1, 2 * jj, TN), v.y, v.x);
-    }
-    if constexpr (SPLIT) {
-      const int jj = e / R, r = e - jj * R;
-      unsigned h0, l0, h1, l1;
-      split_pair(v.x, -v.y, h0, l0);
-      split_pair(v.y, v.x, h1, l1);
-      BwH[(size_t)jj * NT8 + 2 * r] = h0;
-      BwL[(size_t)jj * NT8 + 2 * r] = l0;
-      BwH[(size_t)jj * NT8 + 2 * r + 1] = h1;
-      BwL[(size_t)jj * NT8 + 2 * r + 1] = l1;
     }
   };
 
@@ -898,59 +673,6 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
               dst[2 * q2 + 1] = v1;
             } else {
               st_async2(dst + 2 * q2, (unsigned)(info >> 16), v0, v1, &pready[buf]);
-            }
-          }
-        }
-      }
-    } else if constexpr (SPLIT) {
-      // ---- tensor-core partial products: my 16-row m-tile with all my columns ----
-      // A (factor, bf16 hi/lo words, column-major) x B (next input, [column][n])
-      // on mma.sync m16n8k16: three products hi*hi + hi*lo + lo*hi per k-step
-      float cacc[NT][4];
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) cacc[nt][0] = cacc[nt][1] = cacc[nt][2] = cacc[nt][3] = 0.f;
-      const int g = lane >> 2, t = lane & 3, mb = cw * 16;
-      for (int c = 0; c < nch; ++c, ++idx) {
-        const int slot = (int)(idx % NS);
-        const bool ok = mbar_wait<false>(&full[slot], (unsigned)((idx / NS) & 1), a.err, abort_flag, a.wait_cycles);
-        const uint2* S2 = reinterpret_cast<const uint2*>(ring + (size_t)slot * slot_elems) + mb + g;
-        const int c0 = c * CW;
-        const int nks = (min(CW, nJ - c0) + 7) >> 3;
-        if (ok) {
-          for (int kq = 0; kq < nks; ++kq) {
-            const uint2* pa = S2 + (size_t)(kq * 8 + t) * ldn;
-            const uint2 e0 = pa[0], e1 = pa[8], e2 = pa[4 * (size_t)ldn], e3 = pa[4 * (size_t)ldn + 8];
-            const size_t bo = (size_t)(c0 + kq * 8 + t) * NT8 + g;
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-              const unsigned bh0 = BwH[bo + nt * 8], bh1 = BwH[bo + 4 * NT8 + nt * 8];
-              const unsigned bl0 = BwL[bo + nt * 8], bl1 = BwL[bo + 4 * NT8 + nt * 8];
-              mma_bf16(cacc[nt], e0.x, e1.x, e2.x, e3.x, bh0, bh1);
-              mma_bf16(cacc[nt], e0.x, e1.x, e2.x, e3.x, bl0, bl1);
-              mma_bf16(cacc[nt], e0.y, e1.y, e2.y, e3.y, bh0, bh1);
-            }
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[slot]);
-      }
-      // lane (g, t) holds slot nt*4 + t (real, imaginary) of rows mb+g and mb+g+8:
-      // push each to the CTA that owns the row
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const int sidx = nt * 4 + t;
-        if (sidx < R) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int row = mb + g + 8 * h;
-            if (row < ny) {
-              C v;
-              v.x = cacc[nt][2 * h];
-              v.y = cacc[nt][2 * h + 1];
-              const int info = rowinfo[row];
-              C* dst = Qb + ((size_t)crank * nJcap + (info & 0xffff)) * R + sidx;
-              if (CL == 1) *dst = v;
-              else st_async(dst, (unsigned)(info >> 16), v, &pready[buf]);
             }
           }
         }
@@ -1115,7 +837,7 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
 }
 
 // 16 warps (4 auxiliary + up to 3 row groups x 4 column slices) x 128 registers
-template <typename T, bool SPLIT, bool TCM = false>
+template <typename T, bool TCM = false>
 __global__ void __maxnreg__(128) k_front(FrontArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const DevItem it = a.items[blockIdx.x / (2 * a.cluster)];
@@ -1123,34 +845,31 @@ __global__ void __maxnreg__(128) k_front(FrontArgs a) {
   const int n = it.slot_count;
   if constexpr (TCM) {
     // tensor-core items: 8 or 16 slots (fewer pad with empty slots)
-    if (n <= 8) front_body<T, 8, false, true>(a, it, cl, smem);
-    else front_body<T, 16, false, true>(a, it, cl, smem);
+    if (n <= 8) front_body<T, 8, true>(a, it, cl, smem);
+    else front_body<T, 16, true>(a, it, cl, smem);
   } else if constexpr (sizeof(T) == 4) {
-    if (n <= 1) front_body<T, 1, SPLIT>(a, it, cl, smem);
-    else if (n <= 2) front_body<T, 2, SPLIT>(a, it, cl, smem);
-    else if (n <= 4) front_body<T, 4, SPLIT>(a, it, cl, smem);
-    else if (n <= 8) front_body<T, 8, SPLIT>(a, it, cl, smem);
-    else if (n <= 12) front_body<T, 12, SPLIT>(a, it, cl, smem);
-    else front_body<T, 16, SPLIT>(a, it, cl, smem);
+    if (n <= 1) front_body<T, 1>(a, it, cl, smem);
+    else if (n <= 2) front_body<T, 2>(a, it, cl, smem);
+    else if (n <= 4) front_body<T, 4>(a, it, cl, smem);
+    else if (n <= 8) front_body<T, 8>(a, it, cl, smem);
+    else if (n <= 12) front_body<T, 12>(a, it, cl, smem);
+    else front_body<T, 16>(a, it, cl, smem);
   } else {
-    if (n <= 1) front_body<T, 1, SPLIT>(a, it, cl, smem);
-    else if (n <= 2) front_body<T, 2, SPLIT>(a, it, cl, smem);
-    else if (n <= 4) front_body<T, 4, SPLIT>(a, it, cl, smem);
-    else front_body<T, 8, SPLIT>(a, it, cl, smem);
+    if (n <= 1) front_body<T, 1>(a, it, cl, smem);
+    else if (n <= 2) front_body<T, 2>(a, it, cl, smem);
+    else if (n <= 4) front_body<T, 4>(a, it, cl, smem);
+    else front_body<T, 8>(a, it, cl, smem);
   }
 }
 
 template <typename T>
-size_t smem_need(int ldn_max, int ny_max, int nx_max, int R, int KSW, int CL, int CW, int NS, bool split,
-                 bool tc = false) {
+size_t smem_need(int ldn_max, int ny_max, int nx_max, int R, int KSW, int CL, int CW, int NS, bool tc = false) {
   using C = cx_t<T>;
   const int nJ = (ny_max + CL - 1) / CL + 1;
   // tensor-core items: A stages and the three B terms (+ alignment) instead of the slices' staging
   const size_t tc_bytes = (size_t)kTcStages * 3 * ((ldn_max + 127) / 128) * kTcTile +
                           (size_t)3 * 2 * R * ((2 * nJ + 31) & ~31) * 2 + 128;
-  const size_t staging = split ? 2 * (size_t)(((nJ + 7) & ~7) + 8) * (8 * ((2 * R + 7) / 8)) * sizeof(unsigned)
-                         : tc  ? tc_bytes
-                               : (size_t)KSW * 64 * kMaxRG * R * sizeof(C);
+  const size_t staging = tc ? tc_bytes : (size_t)KSW * 64 * kMaxRG * R * sizeof(C);
   return kHdr + (size_t)NS * CW * ldn_max * sizeof(C) + 4 * (size_t)R * nJ * sizeof(C) + nx_max + nJ + 32 +
          2 * (size_t)CL * R * nJ * sizeof(C) + staging + 4 * (size_t)ny_max +
          2 * (size_t)nx_max * sizeof(C) +
@@ -1165,23 +884,19 @@ namespace {
 // The launch shape of a front: column slices, chunk width and ring depth for
 // R slots on clusters of 2 CL CTAs; false if nothing fits in shared memory.
 template <typename T>
-bool front_shape(int max_ny, int max_nx, int R, int CL, bool split, int maxopt, int* ldn_out, int* ksw_out,
-                 int* cw_out, int* ns_out, size_t* smem_out, bool tc = false) {
-  int ldn = (max_ny + 3) & ~3;
+bool front_shape(int max_ny, int max_nx, int R, int CL, int maxopt, int* ldn_out, int* ksw_out, int* cw_out,
+                 int* ns_out, size_t* smem_out, bool tc = false) {
+  const int ldn = (max_ny + 3) & ~3;
   // tensor-core items: complex64, 8 or 16 slots, at most two 128-row tiles
-  if (tc && (split || sizeof(T) != 4 || (R != 8 && R != 16) || ldn > 256)) return false;
-  if (split) {   // the split factor layout's column stride (4 mod 8)
-    ldn = max_ny;
-    while (ldn % 8 != 4) ++ldn;
-  }
+  if (tc && (sizeof(T) != 4 || (R != 8 && R != 16) || ldn > 256)) return false;
   // largest chunk (columns, multiple of 8, <= ~64 KB) and then the deepest ring that fit
   const int nJmax = (max_ny + CL - 1) / CL;
   // column slices: as many as keep >= 4 columns per slice and the slices'
   // partial-sum staging (KSW x 192 x R) within 64 KB
   int KSW = kMaxKSW;
   // (complex64 with more than 8 slots: two slot groups, so at most 2 slices)
-  const int sgroups = (!split && sizeof(T) == 4 && R > 8) ? 2 : 1;
-  while (KSW > 1 && (split || tc || nJmax < 4 * KSW || KSW * sgroups > kMaxKSW ||
+  const int sgroups = (sizeof(T) == 4 && R > 8) ? 2 : 1;
+  while (KSW > 1 && (tc || nJmax < 4 * KSW || KSW * sgroups > kMaxKSW ||
                      (size_t)KSW * 64 * kMaxRG * R * sizeof(cx_t<T>) > 65536))
     --KSW;
   const int cwmax = (int)std::min<size_t>(((size_t)65536 / ((size_t)ldn * sizeof(cx_t<T>))) & ~size_t(7),
@@ -1189,18 +904,18 @@ bool front_shape(int max_ny, int max_nx, int R, int CL, bool split, int maxopt, 
   int CW = std::max(8, cwmax), NS = 0;
   for (; CW >= 8; CW -= 8) {
     for (NS = 4; NS >= 2; --NS)
-      if (smem_need<T>(ldn, max_ny, max_nx, R, KSW, CL, CW, NS, split, tc) <= (size_t)maxopt) break;
+      if (smem_need<T>(ldn, max_ny, max_nx, R, KSW, CL, CW, NS, tc) <= (size_t)maxopt) break;
     if (NS >= 2) break;
   }
   if (CW < 8) return false;
   *ldn_out = ldn; *ksw_out = KSW; *cw_out = CW; *ns_out = NS;
-  *smem_out = smem_need<T>(ldn, max_ny, max_nx, R, KSW, CL, CW, NS, split, tc);
+  *smem_out = smem_need<T>(ldn, max_ny, max_nx, R, KSW, CL, CW, NS, tc);
   return true;
 }
 
 }  // namespace
 
-int front_fit_mask(bool dbl, bool split, int max_ny, int max_nx, int slots, bool tc) {
+int front_fit_mask(bool dbl, int max_ny, int max_nx, int slots, bool tc) {
   int dev = 0, maxopt = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1208,8 +923,8 @@ int front_fit_mask(bool dbl, bool split, int max_ny, int max_nx, int slots, bool
   int mask = 0, ldn, ksw, cw, ns;
   size_t smem;
   for (int cl = 1; cl <= 4; cl *= 2) {
-    const bool ok = dbl ? front_shape<double>(max_ny, max_nx, R, cl, split, maxopt, &ldn, &ksw, &cw, &ns, &smem, tc)
-                        : front_shape<float>(max_ny, max_nx, R, cl, split, maxopt, &ldn, &ksw, &cw, &ns, &smem, tc);
+    const bool ok = dbl ? front_shape<double>(max_ny, max_nx, R, cl, maxopt, &ldn, &ksw, &cw, &ns, &smem, tc)
+                        : front_shape<float>(max_ny, max_nx, R, cl, maxopt, &ldn, &ksw, &cw, &ns, &smem, tc);
     if (ok) mask |= 1 << cl;
   }
   return mask;
@@ -1220,10 +935,8 @@ cudaError_t launch_front(const FrontArgs& a_in, int max_ny, int max_nx, cudaStre
   if (a_in.item_count <= 0) return cudaSuccess;
   FrontArgs a = a_in;
   const bool dbl = sizeof(T) == 8;
-  const bool split = a.split != 0;
-  if (split && dbl) return cudaErrorInvalidValue;
   const bool tc = a.tc != 0;
-  if (tc && (dbl || split || a.max_slots > 16)) return cudaErrorInvalidValue;
+  if (a.split || (tc && (dbl || a.max_slots > 16))) return cudaErrorInvalidValue;
   const int R = tc ? front_tc_slots(a.max_slots) : std::min(front_rpad(std::max(1, a.max_slots)), front_rmax(dbl));
   if (a.cluster < 1) a.cluster = 1;
   if (a.cluster > 4 || max_nx < 5) return cudaErrorInvalidValue;   // clusters of <= 8; two lines per half
@@ -1232,7 +945,7 @@ cudaError_t launch_front(const FrontArgs& a_in, int max_ny, int max_nx, cudaStre
   cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   int ldn = 0, KSW = 0, CW = 0, NS = 0;
   size_t smem = 0;
-  if (!front_shape<T>(max_ny, max_nx, R, a.cluster, split, maxopt, &ldn, &KSW, &CW, &NS, &smem, tc))
+  if (!front_shape<T>(max_ny, max_nx, R, a.cluster, maxopt, &ldn, &KSW, &CW, &NS, &smem, tc))
     return cudaErrorInvalidConfiguration;
   a.ksw = KSW;
   a.stages = NS;
@@ -1248,10 +961,9 @@ cudaError_t launch_front(const FrontArgs& a_in, int max_ny, int max_nx, cudaStre
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void (*kern)(FrontArgs) = k_front<T, false>;
+  void (*kern)(FrontArgs) = k_front<T>;
   if constexpr (sizeof(T) == 4) {
-    if (split) kern = k_front<float, true>;
-    else if (tc) kern = k_front<float, false, true>;
+    if (tc) kern = k_front<float, true>;
   }
   // the attribute is an upper bound: always the device maximum, so that
   // host threads launching concurrently never lower it under one another
@@ -1279,12 +991,11 @@ int front_max_clusters(bool dbl, int cluster) {
   int n = 0;
   cudaError_t e;
   if (dbl) {
-    cudaFuncSetAttribute(k_front<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt);
-    e = cudaOccupancyMaxActiveClusters(&n, k_front<double, false>, &cfg);
+    cudaFuncSetAttribute(k_front<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt);
+    e = cudaOccupancyMaxActiveClusters(&n, k_front<double>, &cfg);
   } else {
-    cudaFuncSetAttribute(k_front<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt);
-    cudaFuncSetAttribute(k_front<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt);
-    e = cudaOccupancyMaxActiveClusters(&n, k_front<float, false>, &cfg);
+    cudaFuncSetAttribute(k_front<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxopt);
+    e = cudaOccupancyMaxActiveClusters(&n, k_front<float>, &cfg);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
