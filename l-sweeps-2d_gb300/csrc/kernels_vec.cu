@@ -14,24 +14,67 @@ constexpr int kRedBlocks = 1216;   // 8 x 152 SMs
 // globally assembled operator, DDCheckerboard.cpp:2611-2635).  Coefficients are
 // rebuilt from the separable PML profile (one profile serves x and y on the
 // square grid) and the squared slowness: 40 algorithmic bytes per DOF.
-__global__ void k_apply_A(const double2* __restrict__ x, double2* __restrict__ y, int n,
-                          const double2* __restrict__ gp, const double* __restrict__ m, double omega2,
-                          long long n2) {
-  const long long G = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int v = blockIdx.y;
-  if (G >= n2) return;
-  const int gx = (int)(G / n), gy = (int)(G - (long long)gx * n);
-  const double2* xv = x + (long long)v * n2;
-  const double2 lox = gp[gx], hix = gp[n + gx], dgx = gp[2 * n + gx];
+//
+// Bound by FP64 issue (2 FMA per cycle and SM), not by memory: a point costs 22
+// FP64 instructions with complex coefficients and 12 with real ones, and outside
+// the PML the coefficients are real (their imaginary parts are exactly zero, so
+// the sums are the same bits).  A thread owns a y position and walks `rows`
+// x-lines with the three lines' values in registers; NR right-hand sides share
+// the coefficients and the squared slowness.  2102^2 points, four right-hand
+// sides: 0.68 ms with a thread per point and complex arithmetic everywhere, 0.42 ms
+// with this (one right-hand side 0.15 ms, two 0.24).
+constexpr int kAT = 128;   // threads: y positions of a block
+// x == 0 by its bits (a compare would take the FP64 pipe)
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+template <int NR>
+__global__ void __launch_bounds__(kAT) k_apply_A(const double2* __restrict__ x, double2* __restrict__ y, int n,
+                                                 const double2* __restrict__ gp, const double* __restrict__ m,
+                                                 double omega2, long long n2, int rows) {
+  const int gy = blockIdx.x * kAT + threadIdx.x;
+  const int gx0 = blockIdx.y * rows, gx1 = min(n, gx0 + rows);
+  if (gy >= n) return;
+  const int v0 = blockIdx.z * NR;
   const double2 loy = gp[gy], hiy = gp[n + gy], dgy = gp[2 * n + gy];
-  double2 c = cadd(dgx, dgy);
-  c.x -= omega2 * m[G];
-  double2 acc = cmul(c, xv[G]);
-  if (gx > 0) cfma(acc, lox, xv[G - n]);
-  if (gx < n - 1) cfma(acc, hix, xv[G + n]);
-  if (gy > 0) cfma(acc, loy, xv[G - 1]);
-  if (gy < n - 1) cfma(acc, hiy, xv[G + 1]);
-  y[(long long)v * n2 + G] = acc;
+  const bool inner_y = is_zero(loy.y) && is_zero(hiy.y) && is_zero(dgy.y) && gy > 0 && gy < n - 1;
+  const double2* xv[NR];
+  double2 lo[NR], mid[NR];   // x at (gx - 1, gy), (gx, gy)
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    xv[r] = x + (long long)(v0 + r) * n2 + gy;
+    lo[r] = gx0 > 0 ? xv[r][(long long)(gx0 - 1) * n] : make_double2(0.0, 0.0);
+    mid[r] = xv[r][(long long)gx0 * n];
+  }
+  for (int gx = gx0; gx < gx1; ++gx) {
+    const long long G = (long long)gx * n;
+    const double2 lox = gp[gx], hix = gp[n + gx], dgx = gp[2 * n + gx];
+    const double mg = m[G + gy];
+    const double cx = dgx.x + dgy.x - omega2 * mg;
+    // (a branch of whole warps: predicated, both forms would take the FP64 pipe)
+    const bool inner = __all_sync(__activemask(), inner_y && is_zero(lox.y) && is_zero(hix.y) && is_zero(dgx.y) &&
+                                                      gx > 0 && gx < n - 1);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const double2 up = gx < n - 1 ? xv[r][G + n] : make_double2(0.0, 0.0);
+      double2 acc;
+      if (inner) {
+        const double2 a = xv[r][G - 1], b = xv[r][G + 1];
+        acc = make_double2(cx * mid[r].x, cx * mid[r].y);
+        acc.x = fma(lox.x, lo[r].x, acc.x); acc.y = fma(lox.x, lo[r].y, acc.y);
+        acc.x = fma(hix.x, up.x, acc.x);    acc.y = fma(hix.x, up.y, acc.y);
+        acc.x = fma(loy.x, a.x, acc.x);     acc.y = fma(loy.x, a.y, acc.y);
+        acc.x = fma(hiy.x, b.x, acc.x);     acc.y = fma(hiy.x, b.y, acc.y);
+      } else {
+        acc = cmul(make_double2(cx, dgx.y + dgy.y), mid[r]);
+        if (gx > 0) cfma(acc, lox, lo[r]);
+        if (gx < n - 1) cfma(acc, hix, up);
+        if (gy > 0) cfma(acc, loy, xv[r][G - 1]);
+        if (gy < n - 1) cfma(acc, hiy, xv[r][G + 1]);
+      }
+      y[(long long)(v0 + r) * n2 + G + gy] = acc;
+      lo[r] = mid[r];
+      mid[r] = up;
+    }
+  }
 }
 
 // M^-1 x = res1 + (res2 + res3 + res4)  (DDCheckerboard.cpp:733-735)
@@ -204,11 +247,29 @@ inline unsigned nblk(long long n) {
 
 }  // namespace
 
+namespace {
+template <int NR>
+void apply_A_groups(const double2* x, double2* y, int groups, int n, const double2* gprof, const double* mgrid,
+                    double omega2, cudaStream_t st) {
+  // x-lines per thread: a shorter walk reads more of its neighbours' lines twice,
+  // a longer one leaves fewer blocks; the longest that leaves 32 blocks per SM
+  // (2102^2 points, four right-hand sides: 0.47 ms with 8 blocks per SM, 0.42 with 32)
+  const unsigned bx = (unsigned)((n + kAT - 1) / kAT);
+  int rows = 16;
+  while (rows > 2 && (long long)bx * ((n + rows - 1) / rows) * groups < 4 * kRedBlocks) rows /= 2;
+  const dim3 g(bx, (unsigned)((n + rows - 1) / rows), (unsigned)groups);
+  k_apply_A<NR><<<g, kAT, 0, st>>>(x, y, n, gprof, mgrid, omega2, (long long)n * n, rows);
+}
+}  // namespace
+
 cudaError_t launch_apply_A(const double2* x, double2* y, int nrhs, int n_dof, const double2* gprof,
                            const double* mgrid, double omega2, cudaStream_t st) {
   const long long n2 = (long long)n_dof * n_dof;
-  dim3 g((unsigned)((n2 + kVT - 1) / kVT), nrhs);
-  k_apply_A<<<g, kVT, 0, st>>>(x, y, n_dof, gprof, mgrid, omega2, n2);
+  if (nrhs >= 4) apply_A_groups<4>(x, y, nrhs / 4, n_dof, gprof, mgrid, omega2, st);
+  const long long o = (nrhs / 4) * 4 * n2;
+  if (nrhs % 4 == 3) apply_A_groups<3>(x + o, y + o, 1, n_dof, gprof, mgrid, omega2, st);
+  if (nrhs % 4 == 2) apply_A_groups<2>(x + o, y + o, 1, n_dof, gprof, mgrid, omega2, st);
+  if (nrhs % 4 == 1) apply_A_groups<1>(x + o, y + o, 1, n_dof, gprof, mgrid, omega2, st);
   return cudaGetLastError();
 }
 
