@@ -264,12 +264,14 @@ FrontPlan base_plan(const lsw_ctx* ctx) {
   plan.cluster_cap = std::max(1, std::min(4, ctx->max_cluster / 2));
   plan.rmax = front_rmax(dbl);
   plan.csize = dbl ? 16 : 8;
-  if (dbl) { plan.col_cost = 40.0; plan.col_slot_cost = 20.0; }
-  if (ctx->prec == LSW_PREC_SPLIT) {
-    // tensor-core matvec: the per-column cost hardly grows with the slots
-    plan.line_overhead = 2200.0; plan.slot_cost = 0.0; plan.col_cost = 40.0; plan.col_slot_cost = 3.0;
-  }
   plan.sym = sym_factors(ctx);
+  if (plan.sym && ctx->prec == LSW_PREC_SPLIT) {
+    plan.line_overhead = 1200.0; plan.unit_cost = 15.0; plan.unit_slot_cost = 16.0; plan.xchg_cost = 75.0; plan.slot_pad = 4;
+  } else if (plan.sym) {
+    plan.line_overhead = 1440.0; plan.unit_cost = 28.0; plan.unit_slot_cost = 22.0; plan.xchg_cost = 100.0;
+  } else if (dbl) {
+    plan.line_overhead = 2300.0; plan.unit_cost = 0.0; plan.unit_slot_cost = 210.0; plan.xchg_cost = 100.0;
+  }
   for (int cl = 1; cl <= 4; cl *= 2)
     plan.max_clusters[cl] = plan.sym ? sym_max_clusters(ctx->prec == LSW_PREC_SPLIT, 2 * cl)
                                      : front_max_clusters(dbl, 2 * cl);
@@ -312,7 +314,9 @@ lsw_status check_kernel_err(lsw_ctx* ctx, cudaStream_t st);
 
 // ---- sweep-front autotuner ----
 // On the first apply of a batch size the shape of every front -- slots per
-// item (4, 8, 16), CTAs per half chain (1, 2, 4) and, for complex64, line
+// item (1 to 16; a front small enough for items of 1 or 2 only where items of 4
+// leave SMs idle: four right-hand sides on 2 x 2 cells of 128^2, complex64,
+// 1.55 -> 1.14 ms an apply), CTAs per half chain (1, 2, 4) and, for complex64, line
 // products on the CUDA cores or the tensor cores -- is measured on the
 // device: each candidate shape is imposed on every front it fits, each front
 // whose launch is new is run twice and timed the second time with CUDA events
@@ -394,8 +398,9 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
   // per front: (items, max slots, cluster, tensor cores) -> ms
   std::vector<std::map<std::tuple<int, int, int, int>, float>> seen;
   lsw_status s = LSW_OK;
-  for (int r : {4, 8, 16}) {
-    if (r > plan.rmax) continue;
+  for (int r : {1, 2, 4, 8, 16}) {
+    if (r > plan.rmax || r < plan.rmin) continue;
+    if (r < 4 && 16 * nrhs / r > ctx->nsm) continue;   // (no front is small enough: see below)
     for (int cl = 1; cl <= plan.cluster_cap && s == LSW_OK; cl *= 2) {
       if (cl > 1 && plan.max_clusters[cl] <= 0) continue;
       FrontPlan p = plan;
@@ -421,6 +426,9 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
         for (int tc = 0; tc < 2 && s == LSW_OK; ++tc) {
           Front& f = sc.fronts[fi];
           if (f.item_count <= 0 || f.slots_cap != r || f.cluster != cl) continue;   // shape did not fit here
+          // items of one or two slots read the factor more often and pay where
+          // they do not fill the SMs more than twice
+          if (r < 4 && f.item_count > ctx->nsm) continue;
           if (tc && !(tc_candidates(ctx) && tc_fits(ctx, f.max_slots, cl))) continue;
           f.tc = tc != 0;
           const auto shape = std::make_tuple(f.item_count, f.max_slots, f.cluster, tc);
@@ -462,12 +470,18 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
 }
 
 // Per-sweep schedules are tuned as a whole: their launches share the GPU with
-// one another, which a launch timed alone does not show.  For each candidate
-// of the cost model's concurrency (how many launches of its size a per-sweep
-// launch is assumed to share the GPU with: 2, 4, 8) the schedule is built and
-// one whole apply (eager launches on the sweep streams, a zero vector) is
-// timed with CUDA events on the caller's stream after one untimed apply; the
-// entry keeps each candidate's time (r = the candidate, ms = its apply).
+// one another, which a launch timed alone does not show.  Candidates are the
+// cost model's schedules when it assumes that a per-sweep launch shares the GPU
+// with 2, 4 or 8 of its size, and the same shape for every launch, for the
+// shapes with which one step's launches together put half to twice as many CTAs
+// on the device as it has SMs.  Of each, stage 1 and a whole apply (eager
+// launches on the sweep streams, a zero vector) are timed with CUDA events
+// (items of one or two slots spread a small grid's sweeps over the SMs; one
+// vector, 4 x 4 cells of 64^2 in complex128: 11.07 -> 7.78 ms an apply against
+// items of at least four, 4 x 4 of 128^2 in complex64: 3.28 -> 2.58);
+// stage 1 takes its own best shape, then the fastest schedule's stages 2 and 3
+// are each tried with those of the next two.  The entry holds the shape of
+// every launch.
 lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_t st, TuneEntry* out) {
   const auto t_start = std::chrono::steady_clock::now();
   DevBuf tx, ty;
@@ -476,43 +490,108 @@ lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_
   CK(cudaMemsetAsync(tx.p, 0, tx.bytes, st), "memset tuning vector");
   CK(ctx->d_ref.ensure(2 * sizeof(void*)), "cudaMalloc(address table)");
   KL(1, launch_set_refs(reinterpret_cast<const void**>(ctx->d_ref.p), tx.p, ty.p, st), "address table");
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  struct Timed {
+    std::vector<int> r, cl, stage;
+    float t1 = 0.f, rest = 0.f;   // stage 1; the remainder of the apply
+  };
+  cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
   CK(cudaEventCreate(&e0), "cudaEventCreate");
   CK(cudaEventCreate(&e1), "cudaEventCreate");
+  CK(cudaEventCreate(&e2), "cudaEventCreate");
   lsw_status s = LSW_OK;
   bool warm = false;
-  for (int conc : {2, 4, 8}) {
-    FrontPlan p = plan;
-    p.lane_concurrency = conc;
+  std::vector<Timed> all;
+  DevBuf bufs[3];
+  auto measure = [&](const FrontPlan& p) -> lsw_status {
     Schedule sc;
     sc.lanes = true;
     sc.nrhs = nrhs;
-    DevBuf bufs[3];
     std::vector<DevItem> items; std::vector<DevSlot> slots; std::vector<DevGroup> groups;
     try {
       build_schedule(ctx->cells, ctx->N, nrhs, p, ctx->LP, sc.fronts, items, slots, groups, ctx->n2);
     } catch (const std::exception&) {
-      continue;
+      return LSW_OK;
     }
-    if ((s = upload_schedule(ctx, &sc, items, slots, groups, bufs)) != LSW_OK) break;
-    if ((s = ensure_pools(ctx, nrhs, sc.scratch_elems, kLanePlanes)) != LSW_OK) break;
-    float ms = 0.f;
-    for (int rep = warm ? 1 : 0; rep < 2 && s == LSW_OK; ++rep) {
+    Timed t;
+    for (const Front& f : sc.fronts) {
+      t.r.push_back(f.slots_cap); t.cl.push_back(f.cluster); t.stage.push_back(f.stage);
+    }
+    for (const Timed& q : all)
+      if (q.r == t.r && q.cl == t.cl) return LSW_OK;   // measured already
+    lsw_status q;
+    if ((q = upload_schedule(ctx, &sc, items, slots, groups, bufs)) != LSW_OK) return q;
+    if ((q = ensure_pools(ctx, nrhs, sc.scratch_elems, kLanePlanes)) != LSW_OK) return q;
+    for (int rep = warm ? 1 : 0; rep < 2; ++rep) {
       int k = 0;
-      if (cudaEventRecord(e0, st) != cudaSuccess) { s = fail(ctx, LSW_ERR_CUDA, "event"); break; }
-      if ((s = enqueue_apply(ctx, &sc, nrhs, st, &k)) != LSW_OK) break;
-      ctx->launches += k;
-      if (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-          cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)
-        s = fail(ctx, LSW_ERR_CUDA, "timing a per-sweep schedule");
+      float whole = 0.f;
+      CK(cudaEventRecord(e0, st), "event");
+      if ((q = launch_front_of(ctx, &sc, 0, st)) != LSW_OK) return q;
+      CK(cudaEventRecord(e1, st), "event");
+      if ((q = enqueue_apply(ctx, &sc, nrhs, st, &k)) != LSW_OK) return q;
+      ctx->launches += k + 1;
+      CK(cudaEventRecord(e2, st), "event");
+      CK(cudaEventSynchronize(e2), "timing a per-sweep schedule");
+      CK(cudaEventElapsedTime(&t.t1, e0, e1), "timing a per-sweep schedule");
+      CK(cudaEventElapsedTime(&whole, e1, e2), "timing a per-sweep schedule");
+      t.rest = whole - t.t1;
     }
     warm = true;
-    if (s == LSW_OK) s = check_kernel_err(ctx, st);
+    all.push_back(t);
+    return check_kernel_err(ctx, st);
+  };
+  const size_t nl = 16 * (size_t)ctx->N + 16;   // at least the launches of an apply
+  for (int conc : {2, 4, 8}) {
     if (s != LSW_OK) break;
-    out->r.push_back(conc); out->cl.push_back(0); out->tc.push_back(0); out->ms.push_back(ms);
+    FrontPlan p = plan;
+    p.lane_concurrency = conc;
+    s = measure(p);
+  }
+  for (int r : {1, 2, 4, 8, 16})
+    for (int cl = 1; cl <= plan.cluster_cap && s == LSW_OK; cl *= 2) {
+      // one step of the four stage-2 sweeps: N cells of 4 nrhs slots each
+      const long long ctas = 4LL * ctx->N * ((4 * nrhs + r - 1) / r) * 2 * cl;
+      if (r > plan.rmax || r > 4 * nrhs || 2 * ctas < ctx->nsm || ctas > 2 * ctx->nsm) continue;
+      if (cl > 1 && plan.max_clusters[cl] <= 0) continue;
+      FrontPlan p = plan;
+      p.forced_r.assign(nl, r);
+      p.forced_cl.assign(nl, cl);
+      s = measure(p);
+    }
+  if (s == LSW_OK && !all.empty()) {
+    std::vector<size_t> by_rest(all.size());
+    for (size_t i = 0; i < all.size(); ++i) by_rest[i] = i;
+    std::sort(by_rest.begin(), by_rest.end(), [&](size_t a, size_t b) { return all[a].rest < all[b].rest; });
+    size_t one = 0;
+    for (size_t i = 1; i < all.size(); ++i)
+      if (all[i].t1 < all[one].t1) one = i;
+    // stage 2 of one, stage 3 of another, stage 1 of its own best
+    auto mix = [&](size_t two, size_t three) {
+      FrontPlan p = plan;
+      p.forced_r.assign(all[two].r.size(), 0);
+      p.forced_cl.assign(all[two].r.size(), 0);
+      for (size_t i = 0; i < all[two].r.size(); ++i) {
+        const size_t from = all[two].stage[i] == 1 ? one : (all[two].stage[i] == 2 ? two : three);
+        p.forced_r[i] = all[from].r[i];
+        p.forced_cl[i] = all[from].cl[i];
+      }
+      return p;
+    };
+    const size_t b = by_rest[0];
+    s = measure(mix(b, b));
+    for (size_t i = 1; i < by_rest.size() && i < 3 && s == LSW_OK; ++i) {
+      if ((s = measure(mix(b, by_rest[i]))) == LSW_OK) s = measure(mix(by_rest[i], b));
+    }
+    size_t best = 0;
+    for (size_t i = 1; i < all.size(); ++i)
+      if (all[i].t1 + all[i].rest < all[best].t1 + all[best].rest) best = i;
+    out->r = all[best].r;
+    out->cl = all[best].cl;
+    out->tc.assign(out->r.size(), 0);
+    out->ms.assign(out->r.size(), all[best].t1 + all[best].rest);
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  cudaEventDestroy(e2);
   CK(cudaStreamSynchronize(st), "tuning sync");
   ctx->d_scratch.release();
   ctx->tune_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
@@ -532,6 +611,7 @@ lsw_status ensure_batch(lsw_ctx* ctx, int nrhs, Schedule** out, cudaStream_t st)
       return fail(ctx, LSW_ERR_UNSUPPORTED, ex.what());
     }
     plan.lanes = nrhs <= ctx->lanes_max_rhs;
+    plan.rmin = ctx->force_r > 0 ? std::min(ctx->force_r, 4) : (plan.lanes || nrhs > 2 ? 1 : 4);
     TuneEntry tuned;
     if (ctx->force_r > 0) {
       plan.forced_r.assign(16 * (size_t)ctx->N + 16, ctx->force_r);
@@ -539,7 +619,7 @@ lsw_status ensure_batch(lsw_ctx* ctx, int nrhs, Schedule** out, cudaStream_t st)
     } else if (ctx->tune && ctx->factorized && plan.lanes) {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       tune_file_read();
-      const std::string key = tune_key(ctx, nrhs) + "|lanes";
+      const std::string key = tune_key(ctx, nrhs) + "|sweeps";
       auto hit = g_tune_cache.find(key);
       TuneEntry whole;
       if (hit != g_tune_cache.end()) {
@@ -552,10 +632,8 @@ lsw_status ensure_batch(lsw_ctx* ctx, int nrhs, Schedule** out, cudaStream_t st)
           tune_file_append(key, whole);
         }
       }
-      size_t best = 0;
-      for (size_t i = 1; i < whole.ms.size(); ++i)
-        if (whole.ms[i] < whole.ms[best]) best = i;
-      if (!whole.r.empty()) plan.lane_concurrency = whole.r[best];
+      plan.forced_r = whole.r;
+      plan.forced_cl = whole.cl;
     } else if (ctx->tune && ctx->factorized) {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       tune_file_read();
@@ -1000,14 +1078,14 @@ lsw_status lsw_ctx_create(lsw_ctx** out, int device) {
   if (const char* ev = std::getenv("LSW_TUNE")) c->tune = std::atoi(ev) != 0;
   // LSW_SWEEP_TC=1 adds tensor-core line products to the complex64 tuning candidates
   if (const char* ev = std::getenv("LSW_SWEEP_TC")) c->sweep_tc = std::atoi(ev) != 0;
-  // LSW_FRONT_SHAPE=RxC imposes R slots per item (4, 8, 16) and C CTAs per half
+  // LSW_FRONT_SHAPE=RxC imposes R slots per item (1, 2, 4, 8, 16) and C CTAs per half
   // chain (1, 2, 4) on every sweep front where that shape fits (no tuning)
   if (const char* ev = std::getenv("LSW_FRONT_SHAPE")) {
     // (RxCt: with the line products on the tensor cores where they fit, complex64)
     int r = 0, cl = 0;
     char t = 0;
     const int got = std::sscanf(ev, "%dx%d%c", &r, &cl, &t);
-    if (got >= 2 && (r == 4 || r == 8 || r == 16) && (cl == 1 || cl == 2 || cl == 4)) {
+    if (got >= 2 && (r == 1 || r == 2 || r == 4 || r == 8 || r == 16) && (cl == 1 || cl == 2 || cl == 4)) {
       c->force_r = r;
       c->force_cl = cl;
       c->force_tc = got == 3 && t == 't';

@@ -277,8 +277,9 @@ void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const Fr
   // ---- flatten into items ----
   // An item takes whole (rhs, shift) groups while they fit in r slots.  A
   // group holds at most 4 slots (the four sweep directions, or the four
-  // L-sweeps, that reach one cell in one front), and the planner only tries
-  // r >= 4, so no group is split over items: every owned output value and
+  // L-sweeps, that reach one cell in one front; one with per-sweep launches),
+  // and the planner only tries r of at least the front's largest group, so no
+  // group is split over items: every owned output value and
   // every trace line is written by one item per front, in one order, and the
   // apply is deterministic (the output adds need no ordering between items).
   auto flatten = [&](std::vector<SlotSpec>& v, int r, auto&& emit) {
@@ -363,9 +364,17 @@ void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const Fr
     double best_t = 1e300;
     long long best_items = 0;
     // fr_r / fr_cl > 0 restrict the search to that shape
+    // the largest (rhs, shift) group: an item takes groups whole
+    int gmax = 1;
+    for (auto& kv : f)
+      for (size_t i = 0, j = 0; i < kv.second.size(); i = j) {
+        while (j < kv.second.size() && kv.second[j].rhs == kv.second[i].rhs && kv.second[j].shift == kv.second[i].shift)
+          ++j;
+        gmax = std::max(gmax, (int)(j - i));
+      }
     auto search = [&](int fr_r, int fr_cl) {
-      for (int r : {16, 8, 4}) {
-        if (r > plan.rmax) continue;
+      for (int r : {16, 8, 4, 2, 1}) {
+        if (r > plan.rmax || r < gmax || r < plan.rmin) continue;
         if (fr_r > 0 && r != fr_r) continue;
         long long n_items = 0;
         int maxs = 0;
@@ -390,8 +399,11 @@ void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const Fr
           if (!(plan.fit_mask[R] & (1 << cl))) continue;   // shared memory
           const long long n_eff = (long long)std::ceil((double)n_items * conc);
           const long long waves = (n_eff + mc - 1) / mc;
-          const double line = plan.line_overhead + plan.slot_cost * R +
-                              (plan.col_cost + plan.col_slot_cost * R) * ((ny_max + cl - 1) / cl);
+          const double units =
+              plan.sym ? SymTiles::elems(ny_max) / 256.0 / cl : (double)((ny_max + cl - 1) / cl);
+          const double Rp = (R + plan.slot_pad - 1) / plan.slot_pad * plan.slot_pad;
+          const double line = plan.line_overhead + (plan.unit_cost + plan.unit_slot_cost * Rp) * units +
+                              (cl > 1 ? plan.xchg_cost * Rp * cl : 0.0);
           double t = (double)waves * (2.0 * nf + 1.0) * line;
           t = std::max(t, conc * fac_elems * plan.csize / plan.bytes_per_cycle);
           // ties go to fewer items (less factor traffic), then to larger clusters

@@ -154,21 +154,25 @@ constexpr int kLanePlane3[4] = {2, 3, 1, 0};       // BL2TR->up, TR2BL->down, BR
 
 // What the front planner knows about the device: how many clusters of each
 // size (1, 2, 4, 8) are resident at once, and a per-line cost model of the
-// sweep-front kernel fitted to front timings on GB300 over every (slots per
-// item, cluster size) choice of a C2 apply: cycles per line =
-//   line_overhead + slot_cost R + (col_cost + col_slot_cost R) x columns per CTA,
-// with a bandwidth floor (factor bytes / bytes_per_cycle).
+// sweep-front kernels fitted to applies of 2 x 2 to 8 x 8 cells of 128^2 (64^2
+// for complex128) with every launch in one shape, 1 to 8 slots per item on 1,
+// 2 and 4 CTAs per half: cycles per line =
+//   line_overhead + (unit_cost + unit_slot_cost R) U + xchg_cost R CTAs (more than one),
+// U = a CTA's 16 x 16 tiles (symmetric factors) or columns (whole blocks) of
+// the line, with a bandwidth floor (factor bytes / bytes_per_cycle).
 struct FrontPlan {
   // indexed by the CTAs per half (1, 2, 4): resident clusters of twice that many CTAs
   int max_clusters[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   int cluster_cap = 4;       // CTAs per half
   int fit_mask[17] = {0};    // per padded slot count: bit CL set where the launch fits in shared memory
   int rmax = 16;
+  int rmin = 4;              // slots per item: the smallest the cost model may choose
   int csize = 8;             // bytes per complex value of the factors
   double line_overhead = 1800.0;
-  double slot_cost = 250.0;
-  double col_cost = 25.0;
-  double col_slot_cost = 10.0;
+  double unit_cost = 25.0;
+  double unit_slot_cost = 10.0;
+  double xchg_cost = 60.0;
+  int slot_pad = 1;          // R counts in multiples of this (split: the tensor cores' columns)
   double bytes_per_cycle = 3300.0;
   // shapes fixed per front (slots per item, CTAs per half), e.g. by the
   // autotuner; an entry of 0, a missing entry or a shape that does not fit
