@@ -26,8 +26,8 @@
 // the classes: every row of tiles finds about 1 / CL of its tiles there, so
 // the CTAs and, within a CTA, the consumer warps (one per 16 rows) are loaded
 // alike.  A warp forms its rows' partial sums in registers:
-//   complex64: lane = (row, even or odd columns of each tile), FMAs, the two
-//              halves added by one shuffle;
+//   complex64: lane = (row, even or odd columns of each tile), or up to 4 slots
+//              (two rows, every fourth column), FMAs, the parts added by shuffles;
 //   split:     mma.sync m16n8k16, the four products of hi and lo words against
 //              the input's hi and lo words, FP32 accumulation (the fourth, lo x
 //              lo, halves the preconditioner's error: 9e-5 against 2e-4 at 163-
@@ -75,6 +75,13 @@ constexpr int SK_NONE = 99;           // padding slot
 // complex64 line input: values per point, a 16-byte pad at 16 slots so that the
 // two columns a warp reads at once lie in distinct banks
 __host__ __device__ constexpr int sym_xs(int R) { return R == 16 ? 18 : R; }
+// complex64: rows per lane of a tile.  A lane with two rows reads the input for
+// half as many columns, and a 16-byte read costs ~1.5 cycles of the SM's shared
+// memory whether its addresses are two or eight (measured): 8 x 8 cells of
+// 128^2, an apply with 2 slots per item 8.8 -> 8.0 ms, with 4 11.7 -> 11.3; with
+// 8 slots (twice the sums: fewer reads in flight) 4 x 4 cells 13.0 -> 14.1, so
+// there a lane keeps one row.
+__host__ __device__ constexpr int sym_rows(int R) { return R <= 4 ? 2 : 1; }
 
 // elements of a lane: (row, slot) pairs it finishes
 template <int R, bool SPLIT> struct Lane {
@@ -378,12 +385,14 @@ __device__ __forceinline__ void sym_body(const FrontArgs& a, const DevItem& it, 
   for (int q = 0; q < (SPLIT ? 2 : 1); ++q)
     ei[q] = to_c(crcp(row_of(q) < ny ? py[4 * ny + row_of(q)] : make_double2(1.0, 0.0)), czero<C>());
   // Byte offset of my accesses within a tile as it is (base_n) or transposed
-  // (base_t).  complex64: of columns (rows) h + 2 i, i = 0 .. 7, of my row
-  // (column) rho, the i-th by XOR masks.  split: of my ldmatrix row, the
-  // transposed tile with its off-diagonal 8 x 8 blocks exchanged.
-  const unsigned base_n = SPLIT ? (unsigned)(lane * 16) : (unsigned)((h * 16 + (rho ^ (4 * h))) * 8);
+  // (base_t).  complex64: of columns (rows) ch + CS i of my row (column) rho and,
+  // with two rows per lane, of row rho ^ 8, each by XOR masks.  split: of my
+  // ldmatrix row, the transposed tile with its off-diagonal 8 x 8 blocks exchanged.
+  constexpr int TR = sym_rows(R), CS = 2 * TR, NI = 8 / TR;   // rows, column step, columns of a lane
+  const int ch = lane >> (5 - TR);
+  const unsigned base_n = SPLIT ? (unsigned)(lane * 16) : (unsigned)((ch * 16 + (rho ^ (4 * ch))) * 8);
   const unsigned base_t = SPLIT ? (unsigned)(((lane & 7) | ((lane & 8) << 1) | ((lane & 16) >> 1)) * 16)
-                                : (unsigned)((rho * 16 + (SymTiles::swz(rho) ^ h)) * 8);
+                                : (unsigned)((rho * 16 + (SymTiles::swz(rho) ^ ch)) * 8);
   // split: my ldmatrix row of the input, n = lane mod 8 of (real plane, k 0-7),
   // (real, k 8-15), (imaginary, k 0-7), (imaginary, k 8-15): (re, im) of a slot
   // against the real plane, (im, re) against the imaginary one, whose products
@@ -632,10 +641,13 @@ __device__ __forceinline__ void sym_body(const FrontArgs& a, const DevItem& it, 
         own[e] = make_float2(acc[0][nt][i] - acc[1][nt][i], acc[0][nt][i + 1] + acc[1][nt][i + 1]);
       }
     } else {
-      C sum[R];
+      // sum[0]: my row; sum[1] (two rows per lane): row rho ^ 8, which is the row of lane ^ 8
+      C sum[TR][R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) sum[r] = czero<C>();
-      const unsigned char* xh = smem + xb + (unsigned)(h * XS * 8);
+      for (int q = 0; q < TR; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) sum[q][r] = czero<C>();
+      const unsigned char* xh = smem + xb + (unsigned)(ch * XS * 8);
 #pragma unroll 1
       for (int qi = 0; qi < NQ; ++qi) {
         const uint2* tl = tiles + (w * 4 + q_first + qi) * 3;
@@ -645,33 +657,49 @@ __device__ __forceinline__ void sym_body(const FrontArgs& a, const DevItem& it, 
         for (int sb = sb0; sb < nb; sb += 4, ++tl) {
           const uint2 d = *tl;
           const bool tn = (int)d.x < 0;
-          // columns (rows) h + 2 i of the tile: XOR masks of the bits of i
-          // (column 2 i: 256 i bytes, rows swizzled by f(2 i))
+          // columns (rows) ch + CS i of the tile: XOR masks of the bits of i
+          // (column CS i: 128 CS i bytes, rows swizzled by f(CS i)), and of row 8
           const unsigned o = base + (d.x & 0x7fffffffu) + (tn ? base_t : base_n);
-          const unsigned m0 = tn ? 16u : 256u | 64u, m1 = tn ? 32u : 512u | 8u, m2 = tn ? 64u : 1024u | 16u;
+          const unsigned m0 = TR == 2 ? (tn ? 32u : 512u | 8u) : (tn ? 16u : 256u | 64u);
+          const unsigned m1 = TR == 2 ? (tn ? 64u : 1024u | 16u) : (tn ? 32u : 512u | 8u);
+          const unsigned m2 = TR == 2 ? (tn ? 1024u | 16u : 64u) : (tn ? 64u : 1024u | 16u);
           const unsigned char* xp = xh + d.y;
-          C v[8];
+          C v[8];                          // [row][column], or [column]
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = lds_c(o ^ ((i & 1 ? m0 : 0u) ^ (i & 2 ? m1 : 0u) ^ (i & 4 ? m2 : 0u)));
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < NI; ++i) {
             if constexpr (R == 1) {
-              cfma(sum[0], v[i], *reinterpret_cast<const C*>(xp + 2 * i * 8));
+              const C q = *reinterpret_cast<const C*>(xp + CS * i * 8);
+#pragma unroll
+              for (int u = 0; u < TR; ++u) cfma(sum[u][0], v[u * 4 + i], q);
             } else {
 #pragma unroll
               for (int r = 0; r < R; r += 2) {
-                const float4 q = *reinterpret_cast<const float4*>(xp + (2 * i * XS + r) * 8);
-                cfma(sum[r], v[i], make_float2(q.x, q.y));
-                cfma(sum[r + 1], v[i], make_float2(q.z, q.w));
+                const float4 q = *reinterpret_cast<const float4*>(xp + (CS * i * XS + r) * 8);
+#pragma unroll
+                for (int u = 0; u < TR; ++u) {
+                  cfma(sum[u][r], v[u * 4 + i], make_float2(q.x, q.y));
+                  cfma(sum[u][r + 1], v[u * 4 + i], make_float2(q.z, q.w));
+                }
               }
             }
           }
         }
         leave(qi);
       }
+      if constexpr (TR == 2) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          C got;
+          got.x = __shfl_xor_sync(0xffffffffu, sum[1][r].x, 8);
+          got.y = __shfl_xor_sync(0xffffffffu, sum[1][r].y, 8);
+          sum[0][r] = cadd(sum[0][r], got);
+        }
+      }
 #pragma unroll
       for (int e = 0; e < NE; ++e) {
-        const C hi = sum[R > 1 ? RH + e : 0], lo = sum[R > 1 ? e : 0];
+        const C hi = sum[0][R > 1 ? RH + e : 0], lo = sum[0][R > 1 ? e : 0];
         const C keep = h && R > 1 ? hi : lo, give = h || R == 1 ? lo : hi;
         C got;
         got.x = __shfl_xor_sync(0xffffffffu, give.x, 16);
