@@ -40,9 +40,15 @@
 // (cp.async.bulk + mbarrier completion); warps 1-2 prefetch the next line's
 // right-hand side (forward) or stored y_k (backward) into shared memory;
 // warp 3 copies y_k (forward) and x_k (backward) to a per-item scratch; the
-// remaining warps are consumers: a lane owns a row pair of a 64-row group and
-// a warp one of KSW interleaved column slices, accumulating in registers with
-// no cross-lane reduction (complex FP32/FP64 FMAs).
+// remaining warps are consumers, accumulating in registers with no cross-lane
+// reduction.  complex64: a lane owns a row pair of a 64-row group and a warp one
+// of KSW interleaved column slices.  complex128 is bound by the FP64 pipes, whose
+// time a warp takes whether its lanes have rows or not, so the (row, slice) pairs
+// lie one after the other over the lanes of up to 12 warps and KSW is the number
+// of slices that leaves the fewest FP64 warp instructions per scheduler: 89
+// points per line fill 356 of 384 lanes with four slices, where row pairs of
+// 64-row groups filled 43 of 64.  4 x 4 cells of 64^2, an apply of one vector 7.65
+// -> 6.28 ms, one cell solve 0.459 -> 0.414 ms.
 // Line vectors and partial sums are stored [column][slot] so that
 // slot offsets are compile-time constants.  The
 // outputs (owned DOFs, trace lines, cell vectors) are written once per item
@@ -216,7 +222,9 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   // so that a warp keeps at most 8 slots of two rows in registers
   constexpr int SG = (sizeof(T) == 4 && R > 8) ? 2 : 1;
   constexpr int RS = R / SG;
-  const int NCW = TC ? kMaxRG * kMaxKSW : KSW * RG * SG;
+  // complex128: the (row, slice) pairs one after the other over the lanes
+  constexpr bool FLAT = sizeof(T) == 8;
+  const int NCW = TC ? kMaxRG * kMaxKSW : FLAT ? (KSW * ny + 31) >> 5 : KSW * RG * SG;
   const int NCT = NCW * 32;
   const int NSYNC = NCT + 96;           // consumers + 2 helper warps + writer warp
   const int nch = (nJ + CW - 1) / CW;   // chunks per line
@@ -266,8 +274,9 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   const size_t qplane = (size_t)nJcap * R;
   const size_t qbuf = (size_t)CL * qplane;
   p = al16(p + 2 * qbuf * sizeof(C));
-  C* LS = reinterpret_cast<C*>(p);      // [KSW][R][64 RG] the column slices' partial sums, before their sum
-  if (!TC) p = al16(p + (size_t)KSW * 64 * RG * R * sizeof(C));
+  const int LR = FLAT ? ny : 64 * RG;
+  C* LS = reinterpret_cast<C*>(p);      // [KSW][R][LR] the column slices' partial sums, before their sum
+  if (!TC) p = al16(p + (size_t)KSW * LR * R * sizeof(C));
   // tensor-core items: the A stages ([stage][term][tile] 128 x 16 bf16) and the
   // line input as B ([term] TN x Kp bf16, Kp = my columns x 2 rounded to 32)
   const int MT = (ldn + 127) >> 7;
@@ -554,10 +563,11 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
   const int cw = warp - kAux;
   if (cw >= NCW) return;   // idle warp (small cell)
   const int ct = cw * 32 + lane;
-  const int sg = cw / (KSW * RG), rg = (cw / KSW) % RG, ks = cw % KSW;   // FMA matvec: slot group, row group, slice
+  // FMA matvec: slot group, row group, slice
+  const int sg = FLAT ? 0 : cw / (KSW * RG), rg = FLAT ? 0 : (cw / KSW) % RG, ks = FLAT ? ct / ny : cw % KSW;
   const int sb = sg * RS;                                                  // first slot of my slot group
-  const int r0 = rg * 64 + 2 * lane;    // my row pair
-  const bool rows_ok = r0 < ldn;
+  const int r0 = FLAT ? ct - ks * ny : rg * 64 + 2 * lane;                 // my row (FLAT) or row pair
+  const bool rows_ok = FLAT ? ks < KSW : r0 < ldn;
 
   // tensor-core items: entry e = (column, slot) of the next line's input as B
   auto write_bw = [&](int e, C v) {
@@ -693,9 +703,15 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
           constexpr int UNR = (RS <= 4 && sizeof(T) == 4) ? 4 : 2;
   #pragma unroll UNR
           for (int cc = ks; cc < ncol; cc += KSW) {
+            const C* v = V + (size_t)(c0 + cc) * R + sb;
+            if constexpr (FLAT) {
+              const C m = S[(size_t)cc * ldn];
+  #pragma unroll
+              for (int r = 0; r < RS; ++r) cfma(acc0[r], m, v[r]);
+              continue;
+            }
             Pair<T> s;
             s.load(S + (size_t)cc * ldn);
-            const C* v = V + (size_t)(c0 + cc) * R + sb;
   #pragma unroll
             for (int r = 0; r < RS; ++r) {
               const C vr = v[r];
@@ -711,20 +727,24 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
       // row's sum to the CTA that owns the row
       // (rows fastest: a lane's row pair is one 16-byte store per slot for
       // float, and consecutive lanes hit consecutive banks)
-      const int RG64 = 64 * RG;
-      {
+      const int RG64 = LR;
+      if (!FLAT || rows_ok) {
         C* ls = LS + ((size_t)ks * R + sb) * RG64 + r0;
   #pragma unroll
-        for (int r = 0; r < RS; ++r) { ls[(size_t)r * RG64] = acc0[r]; ls[(size_t)r * RG64 + 1] = acc1[r]; }
+        for (int r = 0; r < RS; ++r) {
+          ls[(size_t)r * RG64] = acc0[r];
+          if (!FLAT) ls[(size_t)r * RG64 + 1] = acc1[r];
+        }
       }
-      named_sync(3 + rg, KSW * SG * 32);
+      named_sync(3 + rg, FLAT ? NCT : KSW * SG * 32);
       {
         constexpr int UP = (sizeof(T) == 4 && R % 2 == 0) ? 2 : 1;   // slots per store
         constexpr int NU = R / UP;                                  // stores per row
         const size_t lsplane = (size_t)R * RG64;
-        for (int u = (sg * KSW + ks) * 32 + lane; u < 64 * NU; u += KSW * SG * 32) {
-          const int up = u >> 6, rr = u & 63;   // consecutive lanes take consecutive rows
-          const int row = rg * 64 + rr;
+        const int u0 = FLAT ? ct : (sg * KSW + ks) * 32 + lane, un = FLAT ? ny * NU : 64 * NU;
+        for (int u = u0; u < un; u += FLAT ? NCT : KSW * SG * 32) {
+          // consecutive lanes take consecutive rows
+          const int up = FLAT ? (R == 1 ? 0 : u / ny) : u >> 6, row = FLAT ? u - up * ny : rg * 64 + (u & 63);
           if (row >= ny) continue;
           const C* src = LS + (size_t)up * UP * RG64 + row;
           C v0 = src[0], v1 = UP == 2 ? src[RG64] : czero<C>();
@@ -758,9 +778,9 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
       const int kn = last ? mid : line_k(li + 1);
       const C cp = half == 0 ? wsh[kn] : esh[kn];
       for (int e = ct; e < R * nJ; e += NCT) {
-        C s = czero<C>();
         const C* q = Qb + e;
-        for (int pl = 0; pl < nplane; ++pl, q += qplane) s = cadd(s, *q);
+        C s = *q;
+        for (int pl = 1; pl < nplane; ++pl) s = cadd(s, *(q += qplane));
         Y[e] = s;
         if (!last) {
           C b = H[e];
@@ -788,9 +808,9 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
     } else if (li == nf) {
       // middle: x_m, the first backward input of both halves
       for (int e = ct; e < R * nJ; e += NCT) {
-        C s = czero<C>();
         const C* q = Qb + e;
-        for (int pl = 0; pl < nplane; ++pl, q += qplane) s = cadd(s, *q);
+        C s = *q;
+        for (int pl = 1; pl < nplane; ++pl) s = cadd(s, *(q += qplane));
         Y[e] = s;
         V[e] = s;
         write_bw(e, s);
@@ -799,9 +819,9 @@ __device__ __forceinline__ void front_body(const FrontArgs& a, const DevItem& it
       // backward: x_k = y_k - e_k (S_k^{-1} x_{k+1}) or z_k - w_k (T_k^{-1} x_{k-1})
       const C cn = half == 0 ? esh[k] : wsh[k];
       for (int e = ct; e < R * nJ; e += NCT) {
-        C s = czero<C>();
         const C* q = Qb + e;
-        for (int pl = 0; pl < nplane; ++pl, q += qplane) s = cadd(s, *q);
+        C s = *q;
+        for (int pl = 1; pl < nplane; ++pl) s = cadd(s, *(q += qplane));
         C x = H[e];
         cfms(x, cn, s);
         V[e] = x;
@@ -869,7 +889,7 @@ size_t smem_need(int ldn_max, int ny_max, int nx_max, int R, int KSW, int CL, in
   // tensor-core items: A stages and the three B terms (+ alignment) instead of the slices' staging
   const size_t tc_bytes = (size_t)kTcStages * 3 * ((ldn_max + 127) / 128) * kTcTile +
                           (size_t)3 * 2 * R * ((2 * nJ + 31) & ~31) * 2 + 128;
-  const size_t staging = tc ? tc_bytes : (size_t)KSW * 64 * kMaxRG * R * sizeof(C);
+  const size_t staging = tc ? tc_bytes : (size_t)KSW * (sizeof(T) == 8 ? ny_max : 64 * kMaxRG) * R * sizeof(C);
   return kHdr + (size_t)NS * CW * ldn_max * sizeof(C) + 4 * (size_t)R * nJ * sizeof(C) + nx_max + nJ + 32 +
          2 * (size_t)CL * R * nJ * sizeof(C) + staging + 4 * (size_t)ny_max +
          2 * (size_t)nx_max * sizeof(C) +
@@ -899,6 +919,21 @@ bool front_shape(int max_ny, int max_nx, int R, int CL, int maxopt, int* ldn_out
   while (KSW > 1 && (tc || nJmax < 4 * KSW || KSW * sgroups > kMaxKSW ||
                      (size_t)KSW * 64 * kMaxRG * R * sizeof(cx_t<T>) > 65536))
     --KSW;
+  if (sizeof(T) == 8) {
+    // complex128: the slices with the least FP64 work, in warp instructions per
+    // slot: products (complex multiply-adds of the columns of the warps, four
+    // schedulers of which the fullest counts; without that rounding 89 points took
+    // 3 to 9 warps, 10 % slower than row pairs) and the sum of the slices; at most
+    // the 12 consumer warps, staging within 64 KB
+    long long best = -1;
+    KSW = 1;
+    for (int q = 1; q <= 16 && q * max_ny <= 32 * kMaxRG * kMaxKSW; ++q) {
+      if (q > 1 && (nJmax < 2 * q || (size_t)q * max_ny * R * sizeof(cx_t<T>) > 65536)) break;
+      const long long cost =
+          4LL * ((q * max_ny + 127) / 128 * 4) * ((nJmax + q - 1) / q) + 2LL * (q - 1) * ((max_ny + 31) / 32);
+      if (best < 0 || cost <= best) { best = cost; KSW = q; }
+    }
+  }
   const int cwmax = (int)std::min<size_t>(((size_t)65536 / ((size_t)ldn * sizeof(cx_t<T>))) & ~size_t(7),
                                           (size_t)((nJmax + 7) & ~7));
   int CW = std::max(8, cwmax), NS = 0;
