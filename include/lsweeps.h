@@ -56,8 +56,8 @@ typedef enum lsw_precision {
   LSW_PREC_C64 = 1,  /* complex float factors and applies, FP32 accumulation */
   LSW_PREC_SPLIT = 2 /* complex float applies whose factor products run on the tensor cores:
                         every factor entry stored as two bf16 terms (hi + lo, 8 bytes per
-                        complex value like complex float), three bf16 products per entry
-                        (hi*hi + hi*lo + lo*hi) accumulated in FP32 */
+                        complex value like complex float), four bf16 products per entry
+                        (each of hi, lo by each) accumulated in FP32 */
 } lsw_precision;
 
 typedef enum lsw_gmres_mode {
@@ -106,7 +106,8 @@ typedef struct lsw_apply_profile {
   double front_ms;       /* summed device time of the front kernels */
   double total_ms;       /* device time of the whole apply */
   double alg_bytes;      /* algorithmic bytes of the front kernels: per cell and front
-                            2 F + 4 R nx ny s, F = nx ny^2 s the factor, R its slots */
+                            2 F + 4 R nx ny s, F the factor (nx ny^2 s, or nx ny (ny + 1) / 2 s
+                            where it is kept in symmetric tiles), R its slots */
   double alg_flops;      /* 2 x 8 nx ny^2 R real flops per cell and front */
   double streamed_bytes; /* bytes the items stream: a cell whose slots are split over
                             several items reads its (padded) factor once per item */

@@ -1386,7 +1386,8 @@ lsw_status lsw_apply_precond_profiled(lsw_ctx* ctx, const void* x, void* y, int 
   std::vector<DevItem> items(sc->fronts.empty() ? 0 : sc->fronts.back().item_begin + sc->fronts.back().item_count);
   CK(cudaMemcpy(items.data(), sc->d_items, items.size() * sizeof(DevItem), cudaMemcpyDeviceToHost), "D2H items");
   // algorithmic bytes count each cell's factor once per front (forward and
-  // backward pass) however its slots are split into items; the streamed
+  // backward pass), symmetric ones as their lower halves, however its slots are
+  // split into items; the streamed
   // bytes count every item's pass
   const double cs = (double)csize(ctx->prec);
   double bytes = 0.0, flops = 0.0, streamed = 0.0;
@@ -1400,7 +1401,7 @@ lsw_status lsw_apply_precond_profiled(lsw_ctx* ctx, const void* x, void* y, int 
   for (const auto& st_cells : per_step) {
     for (const auto& kv : st_cells.second) {
       const DevCell& c = ctx->cells[kv.first];
-      const double F = (double)c.nx * c.ny * c.ny * cs;
+      const double F = (double)c.nx * c.ny * (sym_factors(ctx) ? (c.ny + 1) / 2.0 : (double)c.ny) * cs;
       bytes += 2.0 * F + 4.0 * kv.second * (double)c.nx * c.ny * cs;
       flops += 2.0 * 8.0 * (double)c.nx * c.ny * c.ny * kv.second;
       slots += kv.second;

@@ -127,7 +127,8 @@ class Request:
 
 def estimate_bytes(spec: ProblemSpec, precision: str, max_batch: int, restart: int = 30) -> int:
     """Device footprint of a resident operator: the factors of every cell
-    (nx x ny x ldn complex values) plus the per-problem vectors, the Krylov
+    (as nx x ny x ldn complex values: the symmetric tiles of the reduced
+    precisions take about half) plus the per-problem vectors, the Krylov
     basis of a batch and the sweep buffers, with 25 % headroom."""
     cs = 16 if precision in ("c128", "fp64") else 8
     side = spec.m + 6 + 2 * spec.p - 1          # interior cell DOFs per side (the largest)
