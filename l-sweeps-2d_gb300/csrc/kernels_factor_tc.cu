@@ -22,9 +22,12 @@
 //     records f_t (column t at step t), the pivots p_t and 1 / f_t[p_t].
 //     The step is a chain of latencies, so every row forms its reciprocal while
 //     the reduction runs (the candidate hands it on in place of column t), the
-//     rows move in 16-byte accesses, and the block's set-up loops are unrolled
-//     with their loads ahead of their stores: 4 x 4 cells of 128^2 21.6 -> 20.3
-//     ms, 8 x 8 42.0 -> 39.5 ms.
+//     rows move in 16-byte accesses, and the loops around the panel have no
+//     branch between their loads (sums of always 16 terms, with zeros where a
+//     block has fewer): 4 x 4 cells of 128^2 21.6 -> 16.5 ms, 8 x 8 42.0 -> 32.8 ms.
+//     Of 445k cycles per line at 163 points the panels took 160k, u 90k, the set-up
+//     of the line 55k (now 25k), the pivot rows 42k (now 29k).  16 warps instead of 8
+//     (128 registers) made the panel and the write-back slower.
 //   * Every other column then receives the B steps at once.  With
 //     u = M1 g (g the pivot rows, M1 = (D + L)^-1 of the pivots' f values)
 //     the rank-B update of the rows that are not pivots of the block is one
@@ -86,7 +89,8 @@ constexpr int kOffKey = kOffPb + 2 * kB * 4;                       // unsigned [
 constexpr int kOffBar = kOffKey + 64;                              // 3 mbarriers
 constexpr int kOffMisc = kOffBar + 24;                             // abort flag, TMEM address
 constexpr int kOffTab = kOffMisc + 16;                             // unsigned char [4][kSymTilesMax]
-constexpr int kSmem = kOffTab + 4 * kSymTilesMax;
+constexpr int kOffPF = (kOffTab + 4 * kSymTilesMax + 15) & ~15;   // float2 [kB][kB]
+constexpr int kSmem = kOffPF + kB * kB * 8;
 static_assert(kOffF == 86016, "layout");
 static_assert(16 * kMaxRows * 8 <= 3 * kATerm, "unscramble staging tile [16][ldn] fits in the A operand area");
 static_assert(kOffBar % 8 == 0, "mbarrier alignment");
@@ -314,6 +318,7 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
   unsigned* tslot = reinterpret_cast<unsigned*>(smem + kOffMisc + 4);
 
   unsigned char* tab = smem + kOffTab;
+  C* PF = reinterpret_cast<C*>(smem + kOffPF);        // [kB][kB] f_s[p_t], s > t, else 0
   const bool sym = layout != FL_WHOLE;
 
   const double2* px = prof + cl.prof_off;  // lo_x, hi_x, dg_x, lo_y, hi_y, dg_y, off_y, e_y
@@ -341,6 +346,8 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int i = tid; i < kMaxRows; i += kT) pslot[i] = -1;
+  // (rows past a narrow block's pivots meet zeros of M1: they must be finite)
+  for (int i = tid; i < kB * kMaxCols; i += kT) GU[i] = z;
   if (sym && tid < 4 * kSymTilesMax)
     tab[tid] = symt->column[SymTiles::rows(n)][tid / kSymTilesMax][tid % kSymTilesMax];
   tc_fence_before();
@@ -457,13 +464,25 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
       }
       for (int cb = 0; cb < nc; cb += 16) {
         float v[32];
+        // (all loads ahead of their uses; columns past the slice read its last one)
+        C fa[16], fb[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) fa[q] = fb[q] = z;
+        if (live && Fa) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) fa[q] = Fa[(size_t)(c0 + min(cb + q, nc - 1)) * ldn + r];
+        }
+        if (live && Fb) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) fb[q] = Fb[(size_t)(c0 + min(cb + q, nc - 1)) * ldn + r];
+        }
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
           const int cc = cb + q, j = c0 + cc;
           C e = z;
           if (live && cc < nc) {
-            if (Fa) e = cneg(cmul(coupa, Fa[(size_t)j * ldn + r]));
-            if (Fb) cfms(e, coupb, Fb[(size_t)j * ldn + r]);
+            if (Fa) e = cneg(cmul(coupa, fa[q]));
+            if (Fb) cfms(e, coupb, fb[q]);
             if (j == r) e = cadd(e, dr);
             else if (j == r - 1) e = cadd(e, lo);
             else if (j == r + 1) e = cadd(e, hi);
@@ -501,11 +520,13 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
         // unpivoted magnitude, found with one warp reduction) publishes its
         // panel values before the barrier, and after it every thread reads
         // the pivot row from its warp's slot and applies the step itself.
-#pragma unroll
-        for (int t = 0; t < kB; ++t) {
-          if (t >= bt) break;
+        // The registers turn by one column per step (row[q] holds column
+        // (t + q) mod 16), so that one step's code serves all sixteen (as fast as
+        // sixteen unrolled steps).
+#pragma unroll 1
+        for (int t = 0; t < bt; ++t) {
           const int par = t & 1;
-          const C v = row[t];
+          const C v = row[0];
           if (live) Fb_[(size_t)t * kMaxRows + r] = v;
           const C vinv = crcp(v);          // (of every row: while the reduction runs)
           // pivot key: |v|^2 as float bits (monotone for non-negative values) with
@@ -520,7 +541,7 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
             float4* dst = reinterpret_cast<float4*>(rw + warp * kB);
 #pragma unroll
             for (int q = 0; q < kB; q += 2) {
-              const C a = q == t ? vinv : row[q], b = q + 1 == t ? vinv : row[q + 1];
+              const C a = q == 0 ? vinv : row[q], b = row[q + 1];
               dst[q / 2] = make_float4(a.x, a.y, b.x, b.y);
             }
           }
@@ -541,13 +562,13 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
             prow[q] = make_float2(v2.x, v2.y);
             prow[q + 1] = make_float2(v2.z, v2.w);
           }
-          const C inv = prow[t];
+          const C inv = prow[0];
           if (r == p) {
             if (!isfinite(abs2(v))) atomicOr(status, 1);
             mine_used = true;
 #pragma unroll
-            for (int q = 0; q < kB; ++q)
-              if (q < bt) row[q] = (q == t) ? inv : cmul(row[q], inv);
+            for (int q = 1; q < kB; ++q) row[q - 1] = cmul(row[q], inv);
+            row[kB - 1] = inv;
             used[r] = 1;
             piv[k0 + t] = r;
             pbb[t] = r;
@@ -555,12 +576,20 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
           } else if (live) {
             const C vi = cmul(v, inv);
 #pragma unroll
-            for (int q = 0; q < kB; ++q)
-              if (q < bt) {
-                if (q == t) row[q] = cneg(vi);
-                else cfms(row[q], vi, prow[q]);
-              }
+            for (int q = 1; q < kB; ++q) {
+              C x = row[q];
+              cfms(x, vi, prow[q]);
+              row[q - 1] = x;
+            }
+            row[kB - 1] = cneg(vi);
           }
+        }
+#pragma unroll 1
+        for (int t = bt; t < kB; ++t) {   // a narrow panel: the rest of the turn
+          const C v = row[0];
+#pragma unroll
+          for (int q = 1; q < kB; ++q) row[q - 1] = row[q];
+          row[kB - 1] = v;
         }
         if (warp_rows) {
 #pragma unroll
@@ -611,6 +640,10 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
       }
       if (tid < bt) pslot[pbb[tid]] = tid;
       __syncthreads();
+      {
+        const int t = tid / kB, q = tid % kB;
+        PF[tid] = q > t && q < bt ? Fb_[(size_t)q * kMaxRows + pbb[min(t, bt - 1)]] : z;
+      }
       // M1 = (D + L)^-1 (D = diag f_t[p_t], L[t][s] = f_s[p_t], s < t), by the
       // last warp (no matrix row: free while the others write the A operand),
       // lane j solving for column j
@@ -626,21 +659,27 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
             mm[t] = cmul(a, ivb[t]);
           }
         }
-        // (stored after the last, so that the loads above do not wait for stores)
+        // (stored after the last, so that the loads above do not wait for stores;
+        // zeros above the diagonal)
 #pragma unroll
         for (int t = 0; t < kB; ++t)
-          if (t < bt) M1[lane * kB + t] = mm[t];   // transposed: [s][t]
+          if (t < bt) M1[lane * kB + t] = t < lane ? z : mm[t];   // transposed: [s][t]
+      } else if (warp == kT / 32 - 1 && lane < kB) {
+#pragma unroll
+        for (int t = 0; t < kB; ++t) M1[lane * kB + t] = z;       // no such pivot
       }
       // A operand: f_t[r] as (Re, Im) along k, three bf16 terms, one row per
       // thread; zero rows for the block's pivot rows (finished on the CUDA
       // cores after the product) and past the matrix
       if (r < 128 * ntiles) {
-        const bool is_piv = live && pslot[r] >= 0;
+        const bool on = live && pslot[r] < 0;
+        C f[kB];
+#pragma unroll
+        for (int t = 0; t < kB; ++t) f[t] = Fb_[(size_t)min(t, bt - 1) * kMaxRows + min(r, kMaxRows - 1)];
 #pragma unroll
         for (int t = 0; t < kB; ++t) {
-          C f = z;
-          if (live && t < bt && !is_piv) f = Fb_[(size_t)t * kMaxRows + r];
-          put3(Aop, kATerm, kmaj(r, 2 * t), f.x, f.y);
+          const C ft = on && t < bt ? f[t] : z;
+          put3(Aop, kATerm, kmaj(r, 2 * t), ft.x, ft.y);
         }
       }
       // g: the pivot rows of my columns, from the warps that hold them
@@ -672,10 +711,13 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
           const int u = u2 * 2 + (lane >> 4);   // unit: (column quarter-block, pivot quarter)
           const int cc = (u >> 2) * 4 + ((lane >> 2) & 3), t = (u & 3) * 4 + (lane & 3);
           C a = z;
-          if (t < bt && cc < nc && (cc < pcol0 || cc >= pcol1))
+          // (always 16 terms, zeros in M1 where there are fewer: no branch, no bound, so
+          // that all loads are in flight together)
+          const C* m1 = M1 + min(t, bt - 1);
+          const C* gu = GU + min(cc, nc - 1);
 #pragma unroll
-            for (int s2 = 0; s2 < kB; ++s2)
-              if (s2 <= t) cfma(a, M1[s2 * kB + t], GU[(size_t)s2 * kMaxCols + cc]);
+          for (int s2 = 0; s2 < kB; ++s2) cfma(a, m1[s2 * kB], gu[(size_t)s2 * kMaxCols]);
+          if (!(t < bt && cc < nc && (cc < pcol0 || cc >= pcol1))) a = z;
           if (cc < nc) U[(size_t)t * kMaxCols + cc] = a;
           put3(Bop, kBTerm, kmaj(2 * cc, 2 * t), a.x, -a.y);
           put3(Bop, kBTerm, kmaj(2 * cc + 1, 2 * t), a.y, a.x);
@@ -719,10 +761,14 @@ k_factorize_tc(const DevCell* __restrict__ cells, const double2* __restrict__ pr
         const int st_t = issuer / nc, st_c = issuer - (issuer / nc) * nc;
         for (int e = tid; e < bt * nc; e += issuer) {
           C a = U[(size_t)t * kMaxCols + cc];
-          const int pt = pbb[t];
+          const float4* pf = reinterpret_cast<const float4*>(PF + t * kB);
+          const C* us = U + cc;
 #pragma unroll
-          for (int s2 = 1; s2 < kB; ++s2)
-            if (s2 > t && s2 < bt) cfms(a, Fb_[(size_t)s2 * kMaxRows + pt], U[(size_t)s2 * kMaxCols + cc]);
+          for (int s2 = 0; s2 < kB; s2 += 2) {
+            const float4 f2 = pf[s2 / 2];
+            if (s2 > 0) cfms(a, make_float2(f2.x, f2.y), us[(size_t)s2 * kMaxCols]);
+            cfms(a, make_float2(f2.z, f2.w), us[(size_t)(s2 + 1) * kMaxCols]);
+          }
           GU[(size_t)t * kMaxCols + cc] = a;
           t += st_t;
           cc += st_c;
