@@ -50,8 +50,8 @@ DATA = {"C1": "synthetic (constant medium)", "C2": "synthetic (seeded Gaussian-l
         "C3": "synthetic (seeded layered medium)", "C4": "synthetic (seeded piecewise-smooth random medium)"}
 # how L2 is kept out of the timing: every workload streams more factor bytes per apply than L2 holds
 L2_NOTE = {n: f"inputs larger than L2 (129 MB): {gb} of cell factors streamed per preconditioner apply"
-           for n, gb in (("C1", "0.1 GB"), ("C2", "2.3 GB (c64)"), ("C3", "10.7 GB (c64)"),
-                         ("C4", "43.9 GB (bf16x2)"))}
+           for n, gb in (("C1", "0.14 GB with the Krylov basis"), ("C2", "1.2 GB (c64)"),
+                         ("C3", "5.6 GB (c64)"), ("C4", "23.9 GB (bf16x2)"))}
 DTYPE = {"c64": "c64 factors/applies + f64 Krylov",
          "bf16x2": "bf16-split factor products (hi+lo, fp32 accumulate) + f64 Krylov",
          "c128": "c128 factors/applies + f64 Krylov"}

@@ -540,6 +540,8 @@ lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_
     return check_kernel_err(ctx, st);
   };
   const size_t nl = 16 * (size_t)ctx->N + 16;   // at least the launches of an apply
+  // (past a second the model's candidates do: an apply of that size fills the device in any shape)
+  auto spent = [&]() { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count(); };
   for (int conc : {2, 4, 8}) {
     if (s != LSW_OK) break;
     FrontPlan p = plan;
@@ -550,7 +552,7 @@ lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_
     for (int cl = 1; cl <= plan.cluster_cap && s == LSW_OK; cl *= 2) {
       // one step of the four stage-2 sweeps: N cells of 4 nrhs slots each
       const long long ctas = 4LL * ctx->N * ((4 * nrhs + r - 1) / r) * 2 * cl;
-      if (r > plan.rmax || r > 4 * nrhs || 2 * ctas < ctx->nsm || ctas > 2 * ctx->nsm) continue;
+      if (r > plan.rmax || r > 4 * nrhs || 2 * ctas < ctx->nsm || ctas > 2 * ctx->nsm || spent() > 1.0) continue;
       if (cl > 1 && plan.max_clusters[cl] <= 0) continue;
       FrontPlan p = plan;
       p.forced_r.assign(nl, r);
@@ -577,8 +579,8 @@ lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_
       return p;
     };
     const size_t b = by_rest[0];
-    s = measure(mix(b, b));
-    for (size_t i = 1; i < by_rest.size() && i < 3 && s == LSW_OK; ++i) {
+    if (spent() <= 1.0) s = measure(mix(b, b));
+    for (size_t i = 1; i < by_rest.size() && i < 3 && s == LSW_OK && spent() <= 1.0; ++i) {
       if ((s = measure(mix(b, by_rest[i]))) == LSW_OK) s = measure(mix(by_rest[i], b));
     }
     size_t best = 0;
@@ -1241,21 +1243,28 @@ lsw_status lsw_problem_setup(lsw_ctx* ctx, const lsw_geom* g, const double* m_gr
   std::vector<double2> prof;
   long long fac_off = 0;
   ctx->max_nx = ctx->max_ny = 0;
-  for (int I = 0; I < ctx->N; ++I)
+  for (int I = 0; I < ctx->N; ++I) {
+    // the y-profile of a row of cells
+    const DirGeom gy = dir_geom(I, ctx->N, ctx->m, ctx->p);
+    std::vector<double2> yp;
+    {
+      const Profile1D prof_y = make_profile(gy.nel, ctx->p, ctx->h, ctx->C);
+      push_profile(yp, prof_y);
+      if (sym_factors(ctx)) push_symmetrised(yp, prof_y);
+    }
     for (int J = 0; J < ctx->N; ++J) {
       DevCell c = make_cell(I, J, ctx->N, ctx->m, ctx->p, sym_factors(ctx));
       c.fac_off = fac_off;
       fac_off += (long long)c.nx * c.blk;
       c.prof_off = (long long)prof.size();
-      const DirGeom gx = dir_geom(J, ctx->N, ctx->m, ctx->p), gy = dir_geom(I, ctx->N, ctx->m, ctx->p);
+      const DirGeom gx = dir_geom(J, ctx->N, ctx->m, ctx->p);
       push_profile(prof, make_profile(gx.nel, ctx->p, ctx->h, ctx->C));
-      const Profile1D prof_y = make_profile(gy.nel, ctx->p, ctx->h, ctx->C);
-      push_profile(prof, prof_y);
-      push_symmetrised(prof, prof_y);
+      prof.insert(prof.end(), yp.begin(), yp.end());
       ctx->max_nx = std::max(ctx->max_nx, c.nx);
       ctx->max_ny = std::max(ctx->max_ny, c.ny);
       ctx->cells.push_back(c);
     }
+  }
   ctx->LP = ((std::max(ctx->max_nx, ctx->max_ny) + 7) / 8) * 8;
   std::vector<double2> gprof;
   push_profile(gprof, make_profile(ctx->n_g, ctx->p, ctx->h, ctx->C));
@@ -1266,7 +1275,7 @@ lsw_status lsw_problem_setup(lsw_ctx* ctx, const lsw_geom* g, const double* m_gr
   CK(ctx->d_m.ensure((size_t)ctx->n2 * sizeof(double)), "cudaMalloc(m)");
   CK(ctx->d_fac.ensure((size_t)fac_off * cs), "cudaMalloc(factors)");
   CK(ctx->d_status.ensure(16), "cudaMalloc(status)");
-  if (!ctx->d_symt.p) {
+  if (sym_factors(ctx) && !ctx->d_symt.p) {
     static const SymTable symt;
     CK(ctx->d_symt.ensure(sizeof(SymTable)), "cudaMalloc(tile order)");
     CK(cudaMemcpy(ctx->d_symt.p, &symt, sizeof(SymTable), cudaMemcpyHostToDevice), "H2D tile order");

@@ -46,7 +46,7 @@
 // leaving parts out): split 6.6k cycles, of which 3.6k the products (shared-
 // memory reads 2.9k, mma 2.4k) and the rest instructions of one warp after
 // another, ~5 cycles each; complex64 10k, of which 6.6k the products (FMA issue
-// 5k).  Whole blocks took 10.5k and 13.4k.  So the line's code is kept short:
+// 5k; 9.7k with two rows per lane).  Whole blocks took 10.5k and 13.4k.  So the line's code is kept short:
 // addresses precomputed, no branch per tile (predicated loads), nothing built
 // per line that the item can build once.  Two CTAs per SM (72 registers) and
 // sharing an input block among three row tiles were slower.
@@ -106,11 +106,6 @@ __device__ __forceinline__ float2 lds_c(unsigned a) {
 // four 8 x 8 matrices of 16-bit values, lane l giving row l % 8 of matrix l / 8
 __device__ __forceinline__ void ldsm4(unsigned (&r)[4], unsigned addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
-__device__ __forceinline__ void ldsm4_t(unsigned (&r)[4], unsigned addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
 }
