@@ -52,6 +52,8 @@ struct lsw_ctx {
   double h = 0, omega = 0, C = 0;
   long long n2 = 0;
   int max_nx = 0, max_ny = 0, ncell = 0;
+  FrontPlan plan;            // the device's shapes and costs for this problem (cell solves)
+  bool have_plan = false;
   long long LP = 0;
   std::vector<DevCell> cells;
   DevBuf d_symt, d_cells, d_prof, d_gprof, d_m, d_fac, d_work, d_status;
@@ -986,25 +988,44 @@ namespace {
 constexpr size_t kNoAllocScratchBytes = size_t(8) << 20;   // 8 MiB
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
-// scratch of a single-cell solve: elements of an item, bytes of the descriptors
-long long local_item_scratch(const lsw_ctx* ctx, const DevCell& cl, int nrhs, int clus) {
-  return item_scratch(cl, front_rpad(std::min(front_rmax(ctx->prec == LSW_PREC_C128), nrhs)), clus, sym_factors(ctx));
-}
-size_t local_desc_bytes(int nrhs, int rmax) {
-  const size_t items = (nrhs + rmax - 1) / rmax;
+// descriptors of a single-cell solve of `nrhs` right-hand sides in items of r
+size_t local_desc_bytes(int nrhs, int r) {
+  const size_t items = (nrhs + r - 1) / r;
   return (items * sizeof(DevItem) + (size_t)nrhs * sizeof(DevSlot) + 255) & ~size_t(255);
 }
-// CTAs per half of a single-cell solve, the same with and without allocation:
-// one where the x_k rows that several CTAs need would take the scratch past the
-// fixed array
-int local_cluster(const lsw_ctx* ctx, const DevCell& cl, int nrhs) {
-  const int rmax = front_rmax(ctx->prec == LSW_PREC_C128), items = (nrhs + rmax - 1) / rmax;
-  int c = fitting_cluster(ctx, std::min(rmax, nrhs), front_cluster(items, ctx->nsm, ctx->max_cluster));
-  if (sym_factors(ctx) && c > 1 &&
-      local_desc_bytes(nrhs, rmax) + (size_t)items * local_item_scratch(ctx, cl, nrhs, c) * csize(ctx->prec) >
-          kNoAllocScratchBytes)
-    c = fitting_cluster(ctx, std::min(rmax, nrhs), 1);
-  return c;
+// all bytes of such a solve: descriptors and the items' scratch
+size_t local_bytes(const lsw_ctx* ctx, const DevCell& cl, int nrhs, int r, int clus) {
+  const size_t items = (nrhs + r - 1) / r;
+  return local_desc_bytes(nrhs, r) +
+         items * (size_t)item_scratch(cl, front_rpad(std::min(r, nrhs)), clus, sym_factors(ctx)) * csize(ctx->prec);
+}
+// whether the fixed array takes the call: the largest items on one CTA per half
+bool noalloc_fits(const lsw_ctx* ctx, const DevCell& cl, int nrhs) {
+  return local_bytes(ctx, cl, nrhs, front_rmax(ctx->prec == LSW_PREC_C128), 1) <= kNoAllocScratchBytes;
+}
+// Launch shape of a single-cell solve: slots per item and CTAs per half, the
+// same with and without allocation.  Whole blocks: the largest items.  Symmetric
+// tiles: the shape with the fewest cycles by the cost model (cell_solve_shape),
+// of those whose scratch fits in the fixed array where the call as such does.
+struct LocalShape {
+  int r, cl;
+};
+LocalShape local_shape(lsw_ctx* ctx, const DevCell& cl, int nrhs) {
+  const int rmax = front_rmax(ctx->prec == LSW_PREC_C128);
+  if (!sym_factors(ctx))
+    return {rmax, fitting_cluster(ctx, std::min(rmax, nrhs),
+                                  front_cluster((nrhs + rmax - 1) / rmax, ctx->nsm, ctx->max_cluster))};
+  if (!ctx->have_plan) {
+    ctx->plan = base_plan(ctx);
+    ctx->have_plan = true;
+  }
+  const bool bounded = noalloc_fits(ctx, cl, nrhs);
+  const auto fits = [&](int r, int c) {
+    return !bounded || local_bytes(ctx, cl, nrhs, r, c) <= kNoAllocScratchBytes;
+  };
+  LocalShape best{rmax, fitting_cluster(ctx, std::min(rmax, nrhs), 1)};
+  cell_solve_shape(ctx->plan, cl, nrhs, ctx->nsm, fits, &best.r, &best.cl);
+  return best;
 }
 
 // writes the descriptors of `nrhs` full-cell right-hand sides of one cell:
@@ -1229,7 +1250,7 @@ lsw_status lsw_problem_setup(lsw_ctx* ctx, const lsw_geom* g, const double* m_gr
   // drop everything of a previous problem
   ctx->drop_graphs();
   ctx->sched.clear(); ctx->sched_bufs.clear();
-  ctx->is_setup = false; ctx->factorized = false;
+  ctx->is_setup = false; ctx->factorized = false; ctx->have_plan = false;
   ctx->geom = *g;
   ctx->N = g->n_cells; ctx->m = g->n_els_in_cell; ctx->p = g->pml; ctx->h = g->h;
   ctx->n_g = ctx->N * ctx->m + ctx->N - 1;
@@ -1465,13 +1486,12 @@ lsw_status lsw_local_solve(lsw_ctx* ctx, int cell, const void* b, void* x, int n
     return fail(ctx, LSW_ERR_NOT_FACTORIZED, "The linear system has to be factorized before it can be solved");
   CK(cudaSetDevice(ctx->device), "cudaSetDevice");
   cudaStream_t st = S(stream);
-  const bool dbl = ctx->prec == LSW_PREC_C128;
-  const int rmax = front_rmax(dbl);
   const DevCell& cl = ctx->cells[cell];
   std::vector<DevItem> items;
   std::vector<DevSlot> slots;
   long long scr = 0;
-  const int clus = local_cluster(ctx, cl, nrhs);
+  const LocalShape shape = local_shape(ctx, cl, nrhs);
+  const int rmax = shape.r, clus = shape.cl;
   for (int r0 = 0; r0 < nrhs; r0 += rmax) {
     DevItem it{};
     it.cell = cell; it.slot_begin = (int)slots.size(); it.group_begin = 0; it.group_count = 0;
@@ -1925,20 +1945,19 @@ lsw_status lsw_local_solve_noalloc(lsw_ctx* ctx, int cell, const void* b, void* 
     return fail(ctx, LSW_ERR_NOT_FACTORIZED, "The linear system has to be factorized before it can be solved");
   CK(cudaSetDevice(ctx->device), "cudaSetDevice");
   cudaStream_t st = S(stream);
-  const bool dbl = ctx->prec == LSW_PREC_C128;
-  const int rmax = front_rmax(dbl);
   const DevCell& cl = ctx->cells[cell];
-  const int n_items = (nrhs + rmax - 1) / rmax;
-  const int clus = local_cluster(ctx, cl, nrhs);
-  const long long per_item = local_item_scratch(ctx, cl, nrhs, clus);
-  const size_t desc_bytes = local_desc_bytes(nrhs, rmax);
-  const size_t need = desc_bytes + (size_t)n_items * per_item * csize(ctx->prec);
-  if (need > kNoAllocScratchBytes) {
+  if (!noalloc_fits(ctx, cl, nrhs)) {
+    const size_t need = local_bytes(ctx, cl, nrhs, front_rmax(ctx->prec == LSW_PREC_C128), 1);
     return fail(ctx, LSW_ERR_INVALID_ARGUMENT,
                 "lsw_local_solve_noalloc: " + std::to_string(nrhs) + " right-hand sides of cell " +
                     std::to_string(cell) + " need " + std::to_string(need) + " bytes of scratch, more than the " +
                     std::to_string(kNoAllocScratchBytes) + "-byte fixed buffer; use fewer right-hand sides per call");
   }
+  const LocalShape shape = local_shape(ctx, cl, nrhs);
+  const int rmax = shape.r, clus = shape.cl;
+  const int n_items = (nrhs + rmax - 1) / rmax;
+  const long long per_item = item_scratch(cl, front_rpad(std::min(rmax, nrhs)), clus, sym_factors(ctx));
+  const size_t desc_bytes = local_desc_bytes(nrhs, rmax);
   // the array's device address on this context's device (lsw_ctx_create)
   unsigned char* bp = static_cast<unsigned char*>(ctx->noalloc_base);
   if (!bp) return fail(ctx, LSW_ERR_CUDA, "no-allocation scratch address unknown");

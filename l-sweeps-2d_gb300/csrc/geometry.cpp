@@ -117,6 +117,35 @@ DevSlot blank_slot() {
 
 }  // namespace
 
+double line_cycles(const FrontPlan& plan, int R, int cl, int ny) {
+  const double units = plan.sym ? SymTiles::elems(ny) / 256.0 / cl : (double)((ny + cl - 1) / cl);
+  const double Rp = (R + plan.slot_pad - 1) / plan.slot_pad * plan.slot_pad;
+  return plan.line_overhead + (plan.unit_cost + plan.unit_slot_cost * Rp) * units +
+         (cl > 1 ? plan.xchg_cost * Rp * cl : 0.0);
+}
+
+// A cell solve alone leaves most SMs idle, so its right-hand sides go to several
+// items: each streams the factor (from L2, for one cell), but a line costs by its
+// slots.  CTAs per half: as many as put every item on the device at once.  Sixteen
+// right-hand sides, 163 points: as one item complex64 2.59 ms and bf16 split 1.43 ms
+// (whole blocks 1.20 and 0.93), in items of one and four slots 0.28 and 0.36 ms.
+void cell_solve_shape(const FrontPlan& plan, const DevCell& cell, int nrhs, int nsm,
+                      const std::function<bool(int, int)>& fits, int* r, int* cl) {
+  const int nf = cell.nx - 1 - (cell.nx - 1) / 2;
+  double best = 1e300;
+  for (int q : {16, 8, 4, 2, 1}) {
+    if (q > plan.rmax) continue;
+    const int items = (nrhs + q - 1) / q, R = front_rpad(std::min(q, nrhs));
+    int c = front_cluster(items, nsm, 2 * plan.cluster_cap);
+    while (c > 1 && (plan.max_clusters[c] <= 0 || !(plan.fit_mask[R] & (1 << c)) || !fits(q, c))) c /= 2;
+    if (!(plan.fit_mask[R] & (1 << c)) || !fits(q, c)) continue;
+    const int mc = std::max(1, plan.max_clusters[c]), waves = (items + mc - 1) / mc;
+    const double t = std::max(waves * (2.0 * nf + 1.0) * line_cycles(plan, R, c, cell.ny),
+                              items * 2.0 * cell.nx * cell.blk * plan.csize / plan.bytes_per_cycle);
+    if (t < best * 0.98) { best = t; *r = q; *cl = c; }   // (ties: fewer items)
+  }
+}
+
 void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const FrontPlan& plan, long long LP,
                     std::vector<Front>& fronts, std::vector<DevItem>& items, std::vector<DevSlot>& slots,
                     std::vector<DevGroup>& groups, long long n_dof2) {
@@ -399,11 +428,7 @@ void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const Fr
           if (!(plan.fit_mask[R] & (1 << cl))) continue;   // shared memory
           const long long n_eff = (long long)std::ceil((double)n_items * conc);
           const long long waves = (n_eff + mc - 1) / mc;
-          const double units =
-              plan.sym ? SymTiles::elems(ny_max) / 256.0 / cl : (double)((ny_max + cl - 1) / cl);
-          const double Rp = (R + plan.slot_pad - 1) / plan.slot_pad * plan.slot_pad;
-          const double line = plan.line_overhead + (plan.unit_cost + plan.unit_slot_cost * Rp) * units +
-                              (cl > 1 ? plan.xchg_cost * Rp * cl : 0.0);
+          const double line = line_cycles(plan, R, cl, ny_max);
           double t = (double)waves * (2.0 * nf + 1.0) * line;
           t = std::max(t, conc * fac_elems * plan.csize / plan.bytes_per_cycle);
           // ties go to fewer items (less factor traffic), then to larger clusters

@@ -4,6 +4,7 @@
 #include "lsweeps.h"
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 #include <map>
@@ -206,6 +207,13 @@ struct Schedule {
 // sweep, in the order stage 1, stage 2 (t, then sweep), stage 3 (dd, then sweep)).
 // Output groups address the out pool as [rhs][plane][shift] n_dof2 with one
 // plane, or kLanePlanes planes with plan.lanes.
+// cycles per line of items of R slots (padded) on cl CTAs per half, by the cost model
+double line_cycles(const FrontPlan& plan, int R, int cl, int ny);
+// The launch shape (slots per item, CTAs per half) of `nrhs` right-hand sides of
+// one cell on `nsm` SMs, among those that fit in shared memory and that `fits`
+// accepts; *r and *cl stay where there is none.
+void cell_solve_shape(const FrontPlan& plan, const DevCell& cell, int nrhs, int nsm,
+                      const std::function<bool(int, int)>& fits, int* r, int* cl);
 void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const FrontPlan& plan, long long LP,
                     std::vector<Front>& fronts, std::vector<DevItem>& items, std::vector<DevSlot>& slots,
                     std::vector<DevGroup>& groups, long long n_dof2);
