@@ -117,6 +117,27 @@ DevSlot blank_slot() {
 
 }  // namespace
 
+// The slices with the least FP64 work, in warp instructions per slot: products
+// (complex multiply-adds of the columns of the warps, four schedulers of which the
+// fullest counts; without that rounding 89 points took 3 to 9 warps, 10 % slower
+// than row pairs) and the sum of the slices; more than one warp per scheduler where
+// there are enough columns, since one warp waits for its own sums (97 points, one
+// slice: 1.06-1.16x the time of row pairs, two slices 0.87-0.93x; 128 points 1.06-
+// 1.19x and 0.98-1.03x); staging within 64 KB.
+int fp64_slices(int ny, int columns, int R, int lanes) {
+  const auto fits = [&](int q) {
+    return q <= 16 && q * ny <= lanes && (q == 1 || (columns >= 2 * q && (size_t)q * ny * R * 16 <= 65536));
+  };
+  long long best = -1;
+  int slices = 1;
+  for (int q = 1; fits(q); ++q) {
+    if (q * ny <= 128 && fits(q + 1)) continue;
+    const long long cost = 4LL * ((q * ny + 127) / 128 * 4) * ((columns + q - 1) / q) + 2LL * (q - 1) * ((ny + 31) / 32);
+    if (best < 0 || cost <= best) { best = cost; slices = q; }
+  }
+  return slices;
+}
+
 double line_cycles(const FrontPlan& plan, int R, int cl, int ny) {
   const double units = plan.sym ? SymTiles::elems(ny) / 256.0 / cl : (double)((ny + cl - 1) / cl);
   const double Rp = (R + plan.slot_pad - 1) / plan.slot_pad * plan.slot_pad;

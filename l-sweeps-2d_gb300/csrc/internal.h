@@ -207,6 +207,9 @@ struct Schedule {
 // sweep, in the order stage 1, stage 2 (t, then sweep), stage 3 (dd, then sweep)).
 // Output groups address the out pool as [rhs][plane][shift] n_dof2 with one
 // plane, or kLanePlanes planes with plan.lanes.
+// column slices of the complex128 line product: `ny` rows and `columns` columns of
+// a CTA, R slots, on at most `lanes` lanes, a (row, slice) pair each
+int fp64_slices(int ny, int columns, int R, int lanes);
 // cycles per line of items of R slots (padded) on cl CTAs per half, by the cost model
 double line_cycles(const FrontPlan& plan, int R, int cl, int ny);
 // The launch shape (slots per item, CTAs per half) of `nrhs` right-hand sides of

@@ -919,21 +919,7 @@ bool front_shape(int max_ny, int max_nx, int R, int CL, int maxopt, int* ldn_out
   while (KSW > 1 && (tc || nJmax < 4 * KSW || KSW * sgroups > kMaxKSW ||
                      (size_t)KSW * 64 * kMaxRG * R * sizeof(cx_t<T>) > 65536))
     --KSW;
-  if (sizeof(T) == 8) {
-    // complex128: the slices with the least FP64 work, in warp instructions per
-    // slot: products (complex multiply-adds of the columns of the warps, four
-    // schedulers of which the fullest counts; without that rounding 89 points took
-    // 3 to 9 warps, 10 % slower than row pairs) and the sum of the slices; at most
-    // the 12 consumer warps, staging within 64 KB
-    long long best = -1;
-    KSW = 1;
-    for (int q = 1; q <= 16 && q * max_ny <= 32 * kMaxRG * kMaxKSW; ++q) {
-      if (q > 1 && (nJmax < 2 * q || (size_t)q * max_ny * R * sizeof(cx_t<T>) > 65536)) break;
-      const long long cost =
-          4LL * ((q * max_ny + 127) / 128 * 4) * ((nJmax + q - 1) / q) + 2LL * (q - 1) * ((max_ny + 31) / 32);
-      if (best < 0 || cost <= best) { best = cost; KSW = q; }
-    }
-  }
+  if (sizeof(T) == 8) KSW = fp64_slices(max_ny, nJmax, R, 32 * kMaxRG * kMaxKSW);
   const int cwmax = (int)std::min<size_t>(((size_t)65536 / ((size_t)ldn * sizeof(cx_t<T>))) & ~size_t(7),
                                           (size_t)((nJmax + 7) & ~7));
   int CW = std::max(8, cwmax), NS = 0;
