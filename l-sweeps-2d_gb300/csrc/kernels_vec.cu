@@ -21,43 +21,56 @@ constexpr int kRedBlocks = 1216;   // 8 x 152 SMs
 // the sums are the same bits).  A thread owns a y position and walks `rows`
 // x-lines with the three lines' values in registers; NR right-hand sides share
 // the coefficients and the squared slowness.  2102^2 points, four right-hand
-// sides: 0.68 ms with a thread per point and complex arithmetic everywhere, 0.42 ms
-// with this (one right-hand side 0.15 ms, two 0.24).
-constexpr int kAT = 128;   // threads: y positions of a block
+// sides: 0.68 ms with a thread per point and complex arithmetic everywhere, 0.39 ms
+// with this (one right-hand side 0.14 ms, two 0.23).
+//
+// Small grids: as few idle lanes as whole warps allow in y, and down to one x-line
+// per thread.  140^2 points, eight right-hand sides: 15.5 us with blocks of 128 y
+// positions and two lines per thread, 8.9 with this (a thread per point 9.0); 2082^2,
+// four: 415 -> 390 us.
+constexpr int kATMax = 256;   // threads at most: y positions of a block
 // x == 0 by its bits (a compare would take the FP64 pipe)
 __device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+// lines gx0 .. gx1 - 1 of NR right-hand sides
 template <int NR>
-__global__ void __launch_bounds__(kAT) k_apply_A(const double2* __restrict__ x, double2* __restrict__ y, int n,
-                                                 const double2* __restrict__ gp, const double* __restrict__ m,
-                                                 double omega2, long long n2, int rows) {
-  const int gy = blockIdx.x * kAT + threadIdx.x;
-  const int gx0 = blockIdx.y * rows, gx1 = min(n, gx0 + rows);
-  if (gy >= n) return;
-  const int v0 = blockIdx.z * NR;
-  const double2 loy = gp[gy], hiy = gp[n + gy], dgy = gp[2 * n + gy];
+__device__ __forceinline__ void apply_A_lines(const double2* __restrict__ x, double2* __restrict__ y, int n,
+                                              const double2* __restrict__ gp, const double* __restrict__ m,
+                                              double omega2, long long n2, int gy, int gx0, int gx1, int v0) {
+  const double2 loy = gp[gy], hiy = gp[n + gy], dgy = gp[2 * n + gy], zero = make_double2(0.0, 0.0);
   const bool inner_y = is_zero(loy.y) && is_zero(hiy.y) && is_zero(dgy.y) && gy > 0 && gy < n - 1;
   const double2* xv[NR];
   double2 lo[NR], mid[NR];   // x at (gx - 1, gy), (gx, gy)
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     xv[r] = x + (long long)(v0 + r) * n2 + gy;
-    lo[r] = gx0 > 0 ? xv[r][(long long)(gx0 - 1) * n] : make_double2(0.0, 0.0);
+    lo[r] = gx0 > 0 ? xv[r][(long long)(gx0 - 1) * n] : zero;
     mid[r] = xv[r][(long long)gx0 * n];
   }
   for (int gx = gx0; gx < gx1; ++gx) {
     const long long G = (long long)gx * n;
     const double2 lox = gp[gx], hix = gp[n + gx], dgx = gp[2 * n + gx];
     const double mg = m[G + gy];
+    // neighbours of one or two right-hand sides: loaded beside the coefficients that
+    // the branch below waits for
+    double2 ahead[NR <= 2 ? NR : 1][3];
+    if constexpr (NR <= 2) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        ahead[r][0] = gy > 0 ? xv[r][G - 1] : zero;
+        ahead[r][1] = gy < n - 1 ? xv[r][G + 1] : zero;
+        ahead[r][2] = gx < n - 1 ? xv[r][G + n] : zero;
+      }
+    }
     const double cx = dgx.x + dgy.x - omega2 * mg;
     // (a branch of whole warps: predicated, both forms would take the FP64 pipe)
     const bool inner = __all_sync(__activemask(), inner_y && is_zero(lox.y) && is_zero(hix.y) && is_zero(dgx.y) &&
                                                       gx > 0 && gx < n - 1);
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
-      const double2 up = gx < n - 1 ? xv[r][G + n] : make_double2(0.0, 0.0);
+      const double2 up = NR <= 2 ? ahead[r][2] : gx < n - 1 ? xv[r][G + n] : zero;
       double2 acc;
       if (inner) {
-        const double2 a = xv[r][G - 1], b = xv[r][G + 1];
+        const double2 a = NR <= 2 ? ahead[r][0] : xv[r][G - 1], b = NR <= 2 ? ahead[r][1] : xv[r][G + 1];
         acc = make_double2(cx * mid[r].x, cx * mid[r].y);
         acc.x = fma(lox.x, lo[r].x, acc.x); acc.y = fma(lox.x, lo[r].y, acc.y);
         acc.x = fma(hix.x, up.x, acc.x);    acc.y = fma(hix.x, up.y, acc.y);
@@ -67,14 +80,28 @@ __global__ void __launch_bounds__(kAT) k_apply_A(const double2* __restrict__ x, 
         acc = cmul(make_double2(cx, dgx.y + dgy.y), mid[r]);
         if (gx > 0) cfma(acc, lox, lo[r]);
         if (gx < n - 1) cfma(acc, hix, up);
-        if (gy > 0) cfma(acc, loy, xv[r][G - 1]);
-        if (gy < n - 1) cfma(acc, hiy, xv[r][G + 1]);
+        if (gy > 0) cfma(acc, loy, NR <= 2 ? ahead[r][0] : xv[r][G - 1]);
+        if (gy < n - 1) cfma(acc, hiy, NR <= 2 ? ahead[r][1] : xv[r][G + 1]);
       }
       y[(long long)(v0 + r) * n2 + G + gy] = acc;
       lo[r] = mid[r];
       mid[r] = up;
     }
   }
+}
+// groups of NR right-hand sides, the last of NR, NR - 1, NR - 2 or NR - 3
+template <int NR>
+__global__ void __launch_bounds__(kATMax) k_apply_A(const double2* __restrict__ x, double2* __restrict__ y, int n,
+                                                    const double2* __restrict__ gp, const double* __restrict__ m,
+                                                    double omega2, long long n2, int rows, int nrhs) {
+  const int gy = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gx0 = blockIdx.y * rows, gx1 = min(n, gx0 + rows);
+  if (gy >= n) return;
+  const int v0 = blockIdx.z * NR, left = nrhs - v0;
+  if (left >= NR) apply_A_lines<NR>(x, y, n, gp, m, omega2, n2, gy, gx0, gx1, v0);
+  else if (NR > 1 && left == NR - 1) apply_A_lines<(NR > 1 ? NR - 1 : 1)>(x, y, n, gp, m, omega2, n2, gy, gx0, gx1, v0);
+  else if (NR > 2 && left == NR - 2) apply_A_lines<(NR > 2 ? NR - 2 : 1)>(x, y, n, gp, m, omega2, n2, gy, gx0, gx1, v0);
+  else if (NR > 3) apply_A_lines<1>(x, y, n, gp, m, omega2, n2, gy, gx0, gx1, v0);
 }
 
 // M^-1 x = res1 + (res2 + res3 + res4)  (DDCheckerboard.cpp:733-735)
@@ -247,29 +274,35 @@ inline unsigned nblk(long long n) {
 
 }  // namespace
 
-namespace {
-template <int NR>
-void apply_A_groups(const double2* x, double2* y, int groups, int n, const double2* gprof, const double* mgrid,
-                    double omega2, cudaStream_t st) {
-  // x-lines per thread: a shorter walk reads more of its neighbours' lines twice,
-  // a longer one leaves fewer blocks; the longest that leaves 32 blocks per SM
-  // (2102^2 points, four right-hand sides: 0.47 ms with 8 blocks per SM, 0.42 with 32)
-  const unsigned bx = (unsigned)((n + kAT - 1) / kAT);
-  int rows = 16;
-  while (rows > 2 && (long long)bx * ((n + rows - 1) / rows) * groups < 4 * kRedBlocks) rows /= 2;
-  const dim3 g(bx, (unsigned)((n + rows - 1) / rows), (unsigned)groups);
-  k_apply_A<NR><<<g, kAT, 0, st>>>(x, y, n, gprof, mgrid, omega2, (long long)n * n, rows);
-}
-}  // namespace
-
 cudaError_t launch_apply_A(const double2* x, double2* y, int nrhs, int n_dof, const double2* gprof,
                            const double* mgrid, double omega2, cudaStream_t st) {
+  if (nrhs < 1) return cudaSuccess;
   const long long n2 = (long long)n_dof * n_dof;
-  if (nrhs >= 4) apply_A_groups<4>(x, y, nrhs / 4, n_dof, gprof, mgrid, omega2, st);
-  const long long o = (nrhs / 4) * 4 * n2;
-  if (nrhs % 4 == 3) apply_A_groups<3>(x + o, y + o, 1, n_dof, gprof, mgrid, omega2, st);
-  if (nrhs % 4 == 2) apply_A_groups<2>(x + o, y + o, 1, n_dof, gprof, mgrid, omega2, st);
-  if (nrhs % 4 == 1) apply_A_groups<1>(x + o, y + o, 1, n_dof, gprof, mgrid, omega2, st);
+  const int n = n_dof;
+  // the block (whole warps) with the fewest idle lanes in y, of those the one nearest 128
+  int t = 128;
+  long long idle = -1;
+  for (int q : {128, 96, 160, 64, 192, 224, 256}) {
+    const long long w = (long long)((n + q - 1) / q) * q;
+    if (idle < 0 || w < idle) { idle = w; t = q; }
+  }
+  // right-hand sides in groups of at most four, as even as may be, in one launch;
+  // smaller groups where a thread per point and group leaves less than 7 warps per
+  // SM (latency: 64^2 points, four right-hand sides 5.1 us in one group, 2.7 in four)
+  int groups = (nrhs + 3) / 4;
+  while (groups < nrhs && idle * n * groups < 152LL * 7 * 32) groups = std::min(nrhs, 2 * groups);
+  const int nr = (nrhs + groups - 1) / groups;
+  groups = (nrhs + nr - 1) / nr;
+  // x-lines per thread: a shorter walk reads more of its neighbours' lines twice,
+  // a longer one leaves fewer warps; the longest that leaves 128 warps per SM
+  // (2102^2 points, four right-hand sides, blocks of 128: 0.47 ms with 32 warps per SM,
+  // 0.42 with 128)
+  const unsigned bx = (unsigned)((n + t - 1) / t);
+  int rows = 16;
+  while (rows > 1 && (long long)bx * ((n + rows - 1) / rows) * groups * t < 4LL * kRedBlocks * 128) rows /= 2;
+  const dim3 g(bx, (unsigned)((n + rows - 1) / rows), (unsigned)groups);
+  auto* kern = nr == 1 ? k_apply_A<1> : nr == 2 ? k_apply_A<2> : nr == 3 ? k_apply_A<3> : k_apply_A<4>;
+  kern<<<g, t, 0, st>>>(x, y, n, gprof, mgrid, omega2, n2, rows, nrhs);
   return cudaGetLastError();
 }
 
