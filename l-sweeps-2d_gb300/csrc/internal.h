@@ -276,7 +276,8 @@ SymKernel sym_kernel_2(bool split);
 SymKernel sym_kernel_4(bool split);
 // the same front on factors in symmetric tiles (complex64, or bf16 split with a.split)
 cudaError_t launch_front_sym(const FrontArgs& a, int max_ny, int max_nx, cudaStream_t st);
-// clusters of `cluster` CTAs of the sweep-front kernel resident at once (one CTA per SM)
+// clusters of `cluster` CTAs of the sweep-front kernel resident at once, one CTA per SM
+// (those of small cells in symmetric tiles share an SM)
 int front_max_clusters(bool dbl, int cluster);
 int sym_max_clusters(bool split, int cluster);
 int front_rmax(bool dbl);

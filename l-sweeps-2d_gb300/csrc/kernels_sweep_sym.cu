@@ -9,6 +9,11 @@ namespace lsw {
 namespace {
 
 constexpr SymTable kHostTab;
+constexpr int kSmSharedBytes = 233472;   // shared memory of an SM; a CTA takes 1 KB of it besides its own
+// producer and one consumer warp per 16 rows; CTAs of 128 registers per thread
+// that an SM's 64 K registers take
+int sym_warps(int max_ny) { return 1 + (max_ny + 15) / 16; }
+int sym_ctas_per_sm(int max_ny) { return 16 / sym_warps(max_ny); }
 SymKernel sym_kernel(bool split, int cl) {
   return cl == 1 ? sym_kernel_1(split) : cl == 2 ? sym_kernel_2(split) : sym_kernel_4(split);
 }
@@ -28,6 +33,13 @@ int input_bytes(int R, bool split, int n16) {
 // nothing fits.  A chunk is two classes on one or two CTAs per half (a wait and
 // a release per chunk are ~30 instructions of every warp's line), one on four,
 // or the whole line where that is at most 48 KB; two stages at least.
+//
+// Small cells share an SM: a CTA has only the warps of its rows, and the ring only
+// what leaves room for the CTAs that the registers take (a CTA of all twelve rows'
+// warps filled an SM whatever the cell).  An apply of sixteen right-hand sides on
+// 16 x 16 cells of 21 points: complex64 12.6 -> 4.0 ms (whole blocks 10.1), split
+// 12.1 -> 4.5 (10.4); of 53 points 36.2 -> 18.4 (33.6) and 27.3 -> 13.8 (32.0).  Lines of
+// more than 112 points fill an SM as before.
 bool sym_shape(int max_ny, int max_nx, int R, int CL, bool split, int maxopt, int* cpc, int* ns, int* stage,
                size_t* smem) {
   const int nb = (max_ny + 15) / 16, n16 = 16 * nb;
@@ -36,18 +48,22 @@ bool sym_shape(int max_ny, int max_nx, int R, int CL, bool split, int maxopt, in
                        (size_t)(2 * (CL - 1) + 1) * n16 * R * 8 + 2 * (size_t)((max_nx + 1) & ~1) * 8 +
                        kSymTilesMax * 4 * 3 * 8 + (size_t)n16 * 8 + (size_t)((max_nx + 15) & ~15) +
                        (size_t)R * (sizeof(DevSlot) + sizeof(SlotCoef) + sizeof(OutSlot)) + 16;
-  if (fixed >= (size_t)maxopt) return false;
-  const size_t room = (size_t)maxopt - fixed;
+  // as many CTAs per SM as the registers take, fewer where the ring would not fit
   const int nq = 4 / CL;
-  for (int c = nq; c >= 1; c /= 2) {
-    int tiles = 0;
-    for (int q = 0; q < 4; q += c) tiles = std::max(tiles, kHostTab.first[nb][q + c] - kHostTab.first[nb][q]);
-    const size_t st = (size_t)tiles * kTileB;
-    const int n = (int)std::min<size_t>(kRingMax, room / st);
-    if (n < 2 || (c > 2 && st > 49152)) continue;
-    *cpc = c; *ns = n; *stage = (int)st;
-    *smem = fixed + (size_t)n * st;
-    return true;
+  for (int share = sym_ctas_per_sm(max_ny); share >= 1; --share) {
+    const size_t budget = share > 1 ? std::min((size_t)maxopt, (size_t)kSmSharedBytes / share - 1024) : (size_t)maxopt;
+    if (fixed >= budget) continue;
+    const size_t room = budget - fixed;
+    for (int c = nq; c >= 1; c /= 2) {
+      int tiles = 0;
+      for (int q = 0; q < 4; q += c) tiles = std::max(tiles, kHostTab.first[nb][q + c] - kHostTab.first[nb][q]);
+      const size_t st = (size_t)tiles * kTileB;
+      const int n = (int)std::min<size_t>(kRingMax, room / st);
+      if (n < 2 || (c > 2 && st > 49152)) continue;
+      *cpc = c; *ns = n; *stage = (int)st;
+      *smem = fixed + (size_t)n * st;
+      return true;
+    }
   }
   return false;
 }
@@ -82,7 +98,7 @@ cudaError_t launch_front_sym(const FrontArgs& a_in, int max_ny, int max_nx, cuda
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   cfg.gridDim = dim3((unsigned)(a.item_count * 2 * a.cluster));
-  cfg.blockDim = dim3(32 * kSymWarps);
+  cfg.blockDim = dim3(32 * sym_warps(max_ny));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -107,8 +123,8 @@ int sym_max_clusters(bool split, int cluster) {
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   cfg.gridDim = dim3((unsigned)(cluster * 1024));
-  cfg.blockDim = dim3(32 * kSymWarps);
-  cfg.dynamicSmemBytes = (size_t)maxopt;   // one CTA per SM
+  cfg.blockDim = dim3(32 * kSymWarps);     // (the cost model counts one CTA per SM)
+  cfg.dynamicSmemBytes = (size_t)maxopt;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)cluster;
   attr[0].val.clusterDim.y = 1;
