@@ -9,10 +9,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <fstream>
 #include <map>
 #include <stdexcept>
 #include <memory>
 #include <mutex>
+#include <sstream>
 #include <string>
 #include <vector>
 
@@ -342,10 +344,14 @@ std::mutex g_tune_mu;
 std::map<std::string, TuneEntry> g_tune_cache;
 bool g_tune_file_read = false;
 
+// Entries of the cache file hold for the kernels, factor layouts and candidates
+// they were measured with: raise this with any of them.
+constexpr int kTuneRevision = 2;
+
 std::string tune_key(const lsw_ctx* ctx, int nrhs) {
   char b[160];
-  std::snprintf(b, sizeof(b), "|prec%d|N%d|m%d|p%d|rhs%d|cl%d|tc%d", ctx->prec, ctx->N, ctx->m, ctx->p, nrhs,
-                ctx->max_cluster, (int)tc_candidates(ctx));
+  std::snprintf(b, sizeof(b), "|rev%d|prec%d|N%d|m%d|p%d|rhs%d|cl%d|tc%d|tiles%d", kTuneRevision, ctx->prec, ctx->N,
+                ctx->m, ctx->p, nrhs, ctx->max_cluster, (int)tc_candidates(ctx), (int)sym_factors(ctx));
   return ctx->dev_key + b;
 }
 
@@ -354,25 +360,23 @@ void tune_file_read() {
   g_tune_file_read = true;
   const char* path = std::getenv("LSW_TUNE_CACHE");
   if (!path || !*path) return;
-  FILE* f = std::fopen(path, "r");
-  if (!f) return;
-  char line[65536];
-  while (std::fgets(line, sizeof(line), f)) {
-    char* save = nullptr;
-    char* tok = strtok_r(line, " \n", &save);
-    if (!tok) continue;
-    std::string key = tok;
+  std::ifstream f(path);
+  std::string line;
+  // (lines of any length: an entry has a token per launch, per-sweep ones 12 N)
+  while (std::getline(f, line)) {
+    std::istringstream in(line);
+    std::string key, tok;
+    if (!(in >> key)) continue;
     TuneEntry e;
-    while ((tok = strtok_r(nullptr, " \n", &save))) {
+    while (in >> tok) {
       int r = 0, cl = 0;
       float ms = -1.f;
-      if (std::sscanf(tok, "%d,%d,%f", &r, &cl, &ms) != 3) { e.r.clear(); break; }
+      if (std::sscanf(tok.c_str(), "%d,%d,%f", &r, &cl, &ms) != 3) { e.r.clear(); break; }
       // slots per item, + 100 for tensor-core line products
       e.r.push_back(r % 100); e.cl.push_back(cl); e.ms.push_back(ms); e.tc.push_back(r >= 100 ? 1 : 0);
     }
     if (!e.r.empty()) g_tune_cache[key] = e;
   }
-  std::fclose(f);
 }
 
 void tune_file_append(const std::string& key, const TuneEntry& e) {
