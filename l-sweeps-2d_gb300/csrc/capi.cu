@@ -108,6 +108,7 @@ struct lsw_ctx {
   void* noalloc_base = nullptr;
   // optional per-front timing of one apply
   std::vector<cudaEvent_t>* front_events = nullptr;
+  cudaEvent_t stage1_event = nullptr;   // the tuner's, recorded after stage 1 of a per-sweep apply
   // CUDA graphs of the apply, one per batch size, replayed on the caller's
   // stream; a graph is captured against the pools of generation `gen` and
   // captured again when a pool it uses has been reallocated or released
@@ -279,6 +280,8 @@ FrontPlan base_plan(const lsw_ctx* ctx) {
   for (int cl = 1; cl <= 4; cl *= 2)
     plan.max_clusters[cl] = plan.sym ? sym_max_clusters(ctx->prec == LSW_PREC_SPLIT, 2 * cl)
                                      : front_max_clusters(dbl, 2 * cl);
+  // (the tensor-core products of several CTAs on an SM slow one another down)
+  if (plan.sym && ctx->prec == LSW_PREC_C64) plan.ctas_per_sm = sym_ctas_per_sm(ctx->max_ny);
   for (int r = 1; r <= 16; ++r) plan.fit_mask[r] = fit_mask(ctx, r);
   if (plan.max_clusters[1] <= 0) plan.max_clusters[1] = ctx->nsm / 2;
   plan.tc_scratch = ctx->prec == LSW_PREC_C64 && (ctx->sweep_tc || ctx->force_tc);
@@ -476,18 +479,20 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
 }
 
 // Per-sweep schedules are tuned as a whole: their launches share the GPU with
-// one another, which a launch timed alone does not show.  Candidates are the
-// cost model's schedules when it assumes that a per-sweep launch shares the GPU
-// with 2, 4 or 8 of its size, and the same shape for every launch, for the
-// shapes with which one step's launches together put half to twice as many CTAs
-// on the device as it has SMs.  Of each, stage 1 and a whole apply (eager
-// launches on the sweep streams, a zero vector) are timed with CUDA events
-// (items of one or two slots spread a small grid's sweeps over the SMs; one
-// vector, 4 x 4 cells of 64^2 in complex128: 11.07 -> 7.78 ms an apply against
-// items of at least four, 4 x 4 of 128^2 in complex64: 3.28 -> 2.58);
-// stage 1 takes its own best shape, then the fastest schedule's stages 2 and 3
-// are each tried with those of the next two.  The entry holds the shape of
-// every launch.
+// one another, which a launch timed alone does not show.  Four schedules are
+// timed, a whole apply each (eager launches on the sweep streams, a zero vector;
+// twice where it takes less than half a millisecond): the cost model's when it
+// assumes that a per-sweep launch shares the GPU with 2, 4 or 8 of its size, and the
+// shapes that it ranks best for the CTAs of a whole step; then the two mixes of the
+// stages 2 and 3 of the best two.  Stage 1, which runs alone, is that of the schedule
+// where it was fastest.  Which schedules are candidates follows from sizes and the
+// device alone.  (Items of one or two slots spread a small grid's sweeps over the
+// SMs; one vector, 4 x 4 cells of 64^2 in complex128: 11.07 -> 6.2 ms an apply against
+// items of at least four, 4 x 4 of 128^2 in complex64: 3.28 -> 2.43.  A search of up to
+// fourteen schedules, every shape with half to twice as many CTAs in a step as SMs and
+// mixes of the best three, took twice as long over 90 problems; for lines of more
+// than 112 points its applies took the same time in the mean.)  The entry holds the
+// shape of every launch.
 lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_t st, TuneEntry* out) {
   const auto t_start = std::chrono::steady_clock::now();
   DevBuf tx, ty;
@@ -498,16 +503,21 @@ lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_
   KL(1, launch_set_refs(reinterpret_cast<const void**>(ctx->d_ref.p), tx.p, ty.p, st), "address table");
   struct Timed {
     std::vector<int> r, cl, stage;
-    float t1 = 0.f, rest = 0.f;   // stage 1; the remainder of the apply
+    float t1 = 1e30f, rest = 1e30f;   // stage 1; the remainder of the apply
   };
-  cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
-  CK(cudaEventCreate(&e0), "cudaEventCreate");
-  CK(cudaEventCreate(&e1), "cudaEventCreate");
-  CK(cudaEventCreate(&e2), "cudaEventCreate");
+  struct Events {
+    cudaEvent_t e[3] = {nullptr, nullptr, nullptr};
+    ~Events() {
+      for (cudaEvent_t q : e)
+        if (q) cudaEventDestroy(q);
+    }
+  } ev;
+  for (cudaEvent_t& q : ev.e) CK(cudaEventCreate(&q), "cudaEventCreate");
   lsw_status s = LSW_OK;
   bool warm = false;
   std::vector<Timed> all;
   DevBuf bufs[3];
+  // Times the schedule of plan p unless it is one of those timed already.
   auto measure = [&](const FrontPlan& p) -> lsw_status {
     Schedule sc;
     sc.lanes = true;
@@ -523,83 +533,96 @@ lsw_status tune_lanes(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream_
       t.r.push_back(f.slots_cap); t.cl.push_back(f.cluster); t.stage.push_back(f.stage);
     }
     for (const Timed& q : all)
-      if (q.r == t.r && q.cl == t.cl) return LSW_OK;   // measured already
+      if (q.r == t.r && q.cl == t.cl) return LSW_OK;
     lsw_status q;
     if ((q = upload_schedule(ctx, &sc, items, slots, groups, bufs)) != LSW_OK) return q;
     if ((q = ensure_pools(ctx, nrhs, sc.scratch_elems, kLanePlanes)) != LSW_OK) return q;
-    for (int rep = warm ? 1 : 0; rep < 2; ++rep) {
+    // (the first apply of all is not counted)
+    for (int rep = warm ? 0 : -1; rep < 2; ++rep) {
       int k = 0;
-      float whole = 0.f;
-      CK(cudaEventRecord(e0, st), "event");
-      if ((q = launch_front_of(ctx, &sc, 0, st)) != LSW_OK) return q;
-      CK(cudaEventRecord(e1, st), "event");
-      if ((q = enqueue_apply(ctx, &sc, nrhs, st, &k)) != LSW_OK) return q;
-      ctx->launches += k + 1;
-      CK(cudaEventRecord(e2, st), "event");
-      CK(cudaEventSynchronize(e2), "timing a per-sweep schedule");
-      CK(cudaEventElapsedTime(&t.t1, e0, e1), "timing a per-sweep schedule");
-      CK(cudaEventElapsedTime(&whole, e1, e2), "timing a per-sweep schedule");
-      t.rest = whole - t.t1;
+      float t1 = 0.f, rest = 0.f;
+      CK(cudaEventRecord(ev.e[0], st), "event");
+      ctx->stage1_event = ev.e[1];
+      q = enqueue_apply(ctx, &sc, nrhs, st, &k);
+      ctx->stage1_event = nullptr;
+      if (q != LSW_OK) return q;
+      ctx->launches += k;
+      CK(cudaEventRecord(ev.e[2], st), "event");
+      CK(cudaEventSynchronize(ev.e[2]), "timing a per-sweep schedule");
+      CK(cudaEventElapsedTime(&t1, ev.e[0], ev.e[1]), "timing a per-sweep schedule");
+      CK(cudaEventElapsedTime(&rest, ev.e[1], ev.e[2]), "timing a per-sweep schedule");
+      if (rep < 0) continue;
+      t.t1 = std::min(t.t1, t1);
+      t.rest = std::min(t.rest, rest);
+      if (t1 + rest > 0.5f) break;
     }
     warm = true;
     all.push_back(t);
     return check_kernel_err(ctx, st);
   };
-  const size_t nl = 16 * (size_t)ctx->N + 16;   // at least the launches of an apply
-  // (past a second the model's candidates do: an apply of that size fills the device in any shape)
-  auto spent = [&]() { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count(); };
-  for (int conc : {2, 4, 8}) {
-    if (s != LSW_OK) break;
+  // stage 1 as in schedule `one`, stage 2 as in `two`, stage 3 as in `three`
+  auto mix = [&](size_t one, size_t two, size_t three) {
     FrontPlan p = plan;
-    p.lane_concurrency = conc;
-    s = measure(p);
-  }
-  for (int r : {1, 2, 4, 8, 16})
-    for (int cl = 1; cl <= plan.cluster_cap && s == LSW_OK; cl *= 2) {
-      // one step of the four stage-2 sweeps: N cells of 4 nrhs slots each
-      const long long ctas = 4LL * ctx->N * ((4 * nrhs + r - 1) / r) * 2 * cl;
-      if (r > plan.rmax || r > 4 * nrhs || 2 * ctas < ctx->nsm || ctas > 2 * ctx->nsm || spent() > 1.0) continue;
-      if (cl > 1 && plan.max_clusters[cl] <= 0) continue;
-      FrontPlan p = plan;
-      p.forced_r.assign(nl, r);
-      p.forced_cl.assign(nl, cl);
-      s = measure(p);
+    p.forced_r.assign(all[two].r.size(), 0);
+    p.forced_cl.assign(all[two].r.size(), 0);
+    for (size_t i = 0; i < all[two].r.size(); ++i) {
+      const Timed& from = all[all[two].stage[i] == 1 ? one : all[two].stage[i] == 2 ? two : three];
+      p.forced_r[i] = from.r[i];
+      p.forced_cl[i] = from.cl[i];
     }
+    return p;
+  };
+  // candidates: the cost model's (its launches of a step sharing the GPU) and the
+  // shapes that suit the steps of stage 2 (N cells) and of stage 3 (an
+  // anti-diagonal, in the mean)
+  const auto two = lane_shapes(ctx->N, nrhs, ctx->nsm, ctx->max_ny, plan);
+  const auto three = lane_shapes((ctx->N - 1.0) * (ctx->N - 1.0) / std::max(1, 2 * ctx->N - 3), nrhs, ctx->nsm,
+                                 ctx->max_ny, plan);
+  auto fitted = [&](const std::pair<int, int>& a, const std::pair<int, int>& b) {
+    FrontPlan p = plan;
+    // launch 0 is stage 1, then four per step: N - 1 of stage 2, 2 N - 3 of stage 3
+    const size_t n2 = 1 + 4 * (size_t)(ctx->N - 1), n3 = n2 + 4 * (size_t)std::max(0, 2 * ctx->N - 3);
+    for (size_t l = 0; l < n3; ++l) {
+      p.forced_r.push_back(l < n2 ? a.first : b.first);
+      p.forced_cl.push_back(l < n2 ? a.second : b.second);
+    }
+    return p;
+  };
+  std::vector<FrontPlan> tries;
+  auto model = [&](double conc) {
+    tries.push_back(plan);
+    tries.back().lane_concurrency = conc;
+  };
+  model(4);
+  if (!two.empty()) tries.push_back(fitted(two[0], two[0]));
+  if (!two.empty() && !three.empty()) tries.push_back(fitted(two[0], three[0]));
+  model(2);
+  if (two.size() > 1) tries.push_back(fitted(two[1], two[1]));
+  model(8);
+  for (size_t i = 0; i < tries.size() && all.size() < 4 && s == LSW_OK; ++i) s = measure(tries[i]);
   if (s == LSW_OK && !all.empty()) {
-    std::vector<size_t> by_rest(all.size());
-    for (size_t i = 0; i < all.size(); ++i) by_rest[i] = i;
-    std::sort(by_rest.begin(), by_rest.end(), [&](size_t a, size_t b) { return all[a].rest < all[b].rest; });
-    size_t one = 0;
-    for (size_t i = 1; i < all.size(); ++i)
-      if (all[i].t1 < all[one].t1) one = i;
-    // stage 2 of one, stage 3 of another, stage 1 of its own best
-    auto mix = [&](size_t two, size_t three) {
-      FrontPlan p = plan;
-      p.forced_r.assign(all[two].r.size(), 0);
-      p.forced_cl.assign(all[two].r.size(), 0);
-      for (size_t i = 0; i < all[two].r.size(); ++i) {
-        const size_t from = all[two].stage[i] == 1 ? one : (all[two].stage[i] == 2 ? two : three);
-        p.forced_r[i] = all[from].r[i];
-        p.forced_cl[i] = all[from].cl[i];
+    std::vector<size_t> by(all.size());
+    for (size_t i = 0; i < all.size(); ++i) by[i] = i;
+    std::sort(by.begin(), by.end(), [&](size_t a, size_t b) { return all[a].rest < all[b].rest; });
+    size_t one = 0, best = 0;
+    auto pick = [&] {
+      for (size_t i = 0; i < all.size(); ++i) {
+        if (all[i].t1 < all[one].t1) one = i;
+        if (all[i].rest < all[best].rest) best = i;
       }
-      return p;
     };
-    const size_t b = by_rest[0];
-    if (spent() <= 1.0) s = measure(mix(b, b));
-    for (size_t i = 1; i < by_rest.size() && i < 3 && s == LSW_OK && spent() <= 1.0; ++i) {
-      if ((s = measure(mix(b, by_rest[i]))) == LSW_OK) s = measure(mix(by_rest[i], b));
+    pick();
+    if (by.size() > 1) {
+      if ((s = measure(mix(one, by[0], by[1]))) == LSW_OK) s = measure(mix(one, by[1], by[0]));
+      pick();
     }
-    size_t best = 0;
-    for (size_t i = 1; i < all.size(); ++i)
-      if (all[i].t1 + all[i].rest < all[best].t1 + all[best].rest) best = i;
-    out->r = all[best].r;
-    out->cl = all[best].cl;
+    // stage 1 runs alone: the fastest of it and of the rest
+    const FrontPlan p = mix(one, best, best);
+    out->r = p.forced_r;
+    out->cl = p.forced_cl;
     out->tc.assign(out->r.size(), 0);
-    out->ms.assign(out->r.size(), all[best].t1 + all[best].rest);
+    out->ms.assign(out->r.size(), all[one].t1 + all[best].rest);
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaEventDestroy(e2);
   CK(cudaStreamSynchronize(st), "tuning sync");
   ctx->d_scratch.release();
   ctx->tune_seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
@@ -762,6 +785,7 @@ lsw_status enqueue_lanes(lsw_ctx* ctx, Schedule* sc, cudaStream_t st, int* k, bo
     if ((s = launch_front_of(ctx, sc, fi, st)) != LSW_OK) return s;
     *k += sc->fronts[fi].item_count > 0 ? 1 : 0;
   }
+  if (ctx->stage1_event) CK(cudaEventRecord(ctx->stage1_event, st), "event");
   CK(cudaEventRecord(ctx->lane_fork, st), "fork");
   for (int l = 0; l < 8; ++l) CK(cudaStreamWaitEvent(ctx->lane_st[l], ctx->lane_fork, 0), "fork wait");
   int waited[4] = {0, 0, 0, 0};   // per L-sweep: the stage-2 front it last waited for

@@ -167,6 +167,36 @@ void cell_solve_shape(const FrontPlan& plan, const DevCell& cell, int nrhs, int 
   }
 }
 
+std::vector<std::pair<int, int>> lane_shapes(double cells, int nrhs, int nsm, int ny, const FrontPlan& plan) {
+  struct Shape {
+    double t, ctas;
+    int r, cl;
+  };
+  std::vector<Shape> v;
+  for (int r : {1, 2, 4, 8, 16})
+    for (int cl = 1; cl <= plan.cluster_cap; cl *= 2) {
+      const int R = front_rpad(r);
+      if (r > plan.rmax || r < plan.rmin || r > front_rpad(std::min(16, 4 * nrhs)) || !(plan.fit_mask[R] & (1 << cl)) ||
+          (cl > 1 && plan.max_clusters[cl] <= 0))
+        continue;
+      // a step: four sweeps of `cells` cells of 4 nrhs slots each; an exchange carries
+      // no padding
+      const double ctas = 4.0 * cells * ((4 * nrhs + r - 1) / r) * 2 * cl;
+      const double unpadded = cl > 1 ? plan.xchg_cost * ((R + plan.slot_pad - 1) / plan.slot_pad * plan.slot_pad - R) * cl : 0.0;
+      v.push_back({std::ceil(ctas / (nsm * plan.ctas_per_sm)) * (line_cycles(plan, R, cl, ny) - unpadded), ctas, r, cl});
+    }
+  std::vector<std::pair<int, int>> out;
+  while (!v.empty()) {   // the fastest next; of those within 3 % the one of most CTAs, then of fewest per half
+    auto q = std::min_element(v.begin(), v.end(), [](const Shape& a, const Shape& b) { return a.t < b.t; });
+    const double t = q->t;
+    for (auto i = v.begin(); i != v.end(); ++i)
+      if (i->t <= 1.03 * t && (i->ctas > q->ctas || (i->ctas == q->ctas && i->cl < q->cl))) q = i;
+    out.push_back({q->r, q->cl});
+    v.erase(q);
+  }
+  return out;
+}
+
 void build_schedule(const std::vector<DevCell>& cells, int N, int nrhs, const FrontPlan& plan, long long LP,
                     std::vector<Front>& fronts, std::vector<DevItem>& items, std::vector<DevSlot>& slots,
                     std::vector<DevGroup>& groups, long long n_dof2) {

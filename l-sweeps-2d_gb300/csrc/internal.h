@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <functional>
 #include <string>
+#include <utility>
 #include <vector>
 #include <map>
 
@@ -183,6 +184,7 @@ struct FrontPlan {
   // padded): their forward storage is sized for that many slots
   bool tc_scratch = false;
   bool sym = false;          // factors in symmetric tiles
+  int ctas_per_sm = 1;       // CTAs that share an SM without slowing one another down
   // one launch per (step, sweep) instead of one per step (see kLanePlanes);
   // the cost model then counts a stage-2 / stage-3 launch as sharing the GPU
   // with `lane_concurrency` others of its size
@@ -210,6 +212,10 @@ struct Schedule {
 // column slices of the complex128 line product: `ny` rows and `columns` columns of
 // a CTA, R slots, on at most `lanes` lanes, a (row, slice) pair each
 int fp64_slices(int ny, int columns, int R, int lanes);
+// (slots per item, CTAs per half) for a step of the per-sweep launches, `cells`
+// cells in each of the four sweeps, by the cost model's cycles per line times the
+// rounds its CTAs take on `nsm` SMs; the fastest first
+std::vector<std::pair<int, int>> lane_shapes(double cells, int nrhs, int nsm, int ny, const FrontPlan& plan);
 // cycles per line of items of R slots (padded) on cl CTAs per half, by the cost model
 double line_cycles(const FrontPlan& plan, int R, int cl, int ny);
 // The launch shape (slots per item, CTAs per half) of `nrhs` right-hand sides of
@@ -280,6 +286,8 @@ cudaError_t launch_front_sym(const FrontArgs& a, int max_ny, int max_nx, cudaStr
 // (those of small cells in symmetric tiles share an SM)
 int front_max_clusters(bool dbl, int cluster);
 int sym_max_clusters(bool split, int cluster);
+// CTAs of the symmetric-tile kernel that share an SM, by registers
+int sym_ctas_per_sm(int max_ny);
 int front_rmax(bool dbl);
 int front_rpad(int n);
 // bit CL (1, 2, 4) set where items of `slots` slots on clusters of 2 CL CTAs fit in shared memory

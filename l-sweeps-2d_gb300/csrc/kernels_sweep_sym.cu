@@ -10,10 +10,8 @@ namespace {
 
 constexpr SymTable kHostTab;
 constexpr int kSmSharedBytes = 233472;   // shared memory of an SM; a CTA takes 1 KB of it besides its own
-// producer and one consumer warp per 16 rows; CTAs of 128 registers per thread
-// that an SM's 64 K registers take
+// producer and one consumer warp per 16 rows
 int sym_warps(int max_ny) { return 1 + (max_ny + 15) / 16; }
-int sym_ctas_per_sm(int max_ny) { return 16 / sym_warps(max_ny); }
 SymKernel sym_kernel(bool split, int cl) {
   return cl == 1 ? sym_kernel_1(split) : cl == 2 ? sym_kernel_2(split) : sym_kernel_4(split);
 }
@@ -69,6 +67,9 @@ bool sym_shape(int max_ny, int max_nx, int R, int CL, bool split, int maxopt, in
 }
 
 }  // namespace
+
+// (128 registers per thread of an SM's 64 K)
+int sym_ctas_per_sm(int max_ny) { return std::max(1, 16 / (1 + (max_ny + 15) / 16)); }
 
 int sym_fit_mask(bool split, int max_ny, int max_nx, int slots) {
   int dev = 0, maxopt = 0;
