@@ -404,12 +404,15 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0), "cudaEventCreate");
   CK(cudaEventCreate(&e1), "cudaEventCreate");
-  // per front: (items, max slots, cluster, tensor cores) -> ms
+  // per kind of front: (items, max slots, cluster, tensor cores) -> ms.  Fronts with
+  // cells of the same sizes and slot counts (all columns but the last) are one kind and
+  // timed once: 16 x 16 cells of 64^2, four right-hand sides, complex64, 0.99 -> 0.60 s
   std::vector<std::map<std::tuple<int, int, int, int>, float>> seen;
+  std::map<std::vector<std::tuple<int, int, int>>, size_t> kinds;
   lsw_status s = LSW_OK;
   for (int r : {1, 2, 4, 8, 16}) {
     if (r > plan.rmax || r < plan.rmin) continue;
-    if (r < 4 && 16 * nrhs / r > ctx->nsm) continue;   // (no front is small enough: see below)
+    if (r < 4 && 16 * nrhs / r > ctx->nsm * plan.ctas_per_sm) continue;   // (no front is small enough: see below)
     for (int cl = 1; cl <= plan.cluster_cap && s == LSW_OK; cl *= 2) {
       if (cl > 1 && plan.max_clusters[cl] <= 0) continue;
       FrontPlan p = plan;
@@ -429,21 +432,32 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
         out->cl.assign(sc.fronts.size(), 0);
         out->tc.assign(sc.fronts.size(), 0);
         out->ms.assign(sc.fronts.size(), 1e30f);
-        seen.assign(sc.fronts.size(), {});
       }
+      std::vector<size_t> kind(sc.fronts.size());
+      for (size_t fi = 0; fi < sc.fronts.size(); ++fi) {
+        const Front& f = sc.fronts[fi];
+        std::map<int, int> per_cell;
+        for (int i = f.item_begin; i < f.item_begin + f.item_count; ++i) per_cell[items[i].cell] += items[i].slot_count;
+        std::vector<std::tuple<int, int, int>> sizes{std::make_tuple(f.stage, 0, 0)};
+        for (const auto& kv : per_cell)
+          sizes.push_back(std::make_tuple(ctx->cells[kv.first].nx, ctx->cells[kv.first].ny, kv.second));
+        std::sort(sizes.begin() + 1, sizes.end());
+        kind[fi] = kinds.emplace(std::move(sizes), kinds.size()).first->second;
+      }
+      seen.resize(kinds.size());
       for (size_t fi = 0; fi < sc.fronts.size() && s == LSW_OK; ++fi) {
         for (int tc = 0; tc < 2 && s == LSW_OK; ++tc) {
           Front& f = sc.fronts[fi];
           if (f.item_count <= 0 || f.slots_cap != r || f.cluster != cl) continue;   // shape did not fit here
           // items of one or two slots read the factor more often and pay where
-          // they do not fill the SMs more than twice
-          if (r < 4 && f.item_count > ctx->nsm) continue;
+          // they do not fill the SMs more than twice, or their clusters four times
+          if (r < 4 && f.item_count * std::max(2, cl) > 2 * ctx->nsm * plan.ctas_per_sm) continue;
           if (tc && !(tc_candidates(ctx) && tc_fits(ctx, f.max_slots, cl))) continue;
           f.tc = tc != 0;
           const auto shape = std::make_tuple(f.item_count, f.max_slots, f.cluster, tc);
           float ms = 0.f;
-          auto hit = seen[fi].find(shape);
-          if (hit != seen[fi].end()) {
+          auto hit = seen[kind[fi]].find(shape);
+          if (hit != seen[kind[fi]].end()) {
             ms = hit->second;
           } else {
             // timed once; a short launch (where a first launch's overheads
@@ -452,6 +466,7 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
               float t = 0.f;
               if (cudaEventRecord(e0, st) != cudaSuccess) { s = fail(ctx, LSW_ERR_CUDA, "event"); break; }
               if ((s = launch_front_of(ctx, &sc, fi, st)) != LSW_OK) break;
+              ctx->launches += 1;
               if (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
                   cudaEventElapsedTime(&t, e0, e1) != cudaSuccess) {
                 s = fail(ctx, LSW_ERR_CUDA, "timing a sweep-front shape");
@@ -461,7 +476,7 @@ lsw_status tune_fronts(lsw_ctx* ctx, int nrhs, const FrontPlan& plan, cudaStream
               if (t > 2.0f) break;
             }
             if (s != LSW_OK) break;
-            seen[fi][shape] = ms;
+            seen[kind[fi]][shape] = ms;
           }
           if (ms < out->ms[fi] * 0.99f) { out->ms[fi] = ms; out->r[fi] = r; out->cl[fi] = cl; out->tc[fi] = tc; }
         }
@@ -642,6 +657,10 @@ lsw_status ensure_batch(lsw_ctx* ctx, int nrhs, Schedule** out, cudaStream_t st)
       return fail(ctx, LSW_ERR_UNSUPPORTED, ex.what());
     }
     plan.lanes = nrhs <= ctx->lanes_max_rhs;
+    // items of one and two slots: per sweep, and per step for three right-hand sides and
+    // more.  One or two right-hand sides run per step only where per-sweep launches were
+    // turned down, and keep items of four or more there, the shapes that such callers
+    // (and their cached entries) have always had.
     plan.rmin = ctx->force_r > 0 ? std::min(ctx->force_r, 4) : (plan.lanes || nrhs > 2 ? 1 : 4);
     TuneEntry tuned;
     if (ctx->force_r > 0) {

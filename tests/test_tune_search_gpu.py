@@ -60,3 +60,19 @@ def test_search_is_bounded(N, m, p, nrhs, prec):
         first, later = out[p_ + "_tuned"]
         assert later < first <= 2 + (2 + (13 if twice else 7)) * later, (p_, out)
         assert out[p_][0] == out[p_][1]
+
+
+@pytest.mark.parametrize("N,nrhs,prec", [(16, 3, "c64"), (8, 4, "bf16x2"), (6, 5, "c128")])
+def test_fronts_of_one_kind_are_measured_once(N, nrhs, prec):
+    """One launch per step: of the N - 1 columns all but the last are alike (it has the
+    cells of both edges; an odd N has a middle one, too), and are measured once: they
+    hold the same time and shape."""
+    from lsweeps.problems import small
+    from lsweeps.solver import Solver
+    spec, med = small(N=N, m=6, p=2, medium="layered", seed=4)
+    S = Solver(spec, med, precision=prec)
+    S.factorize()
+    fronts = [(f["tuned_ms"], f["slots_cap"], f["cluster"], f["items"]) for f in S.front_shapes(nrhs)[0]]
+    assert len(fronts) == 1 + (N - 1) + (2 * N - 3) and all(f[0] > 0 for f in fronts)
+    assert len(set(fronts[1:N - 1])) == 1
+    S.close()
