@@ -126,17 +126,30 @@ class Request:
 
 
 def estimate_bytes(spec: ProblemSpec, precision: str, max_batch: int, restart: int = 30) -> int:
-    """Device footprint of a resident operator: the factors of every cell
-    (as nx x ny x ldn complex values: the symmetric tiles of the reduced
-    precisions take about half) plus the per-problem vectors, the Krylov
-    basis of a batch and the sweep buffers, with 25 % headroom."""
-    cs = 16 if precision in ("c128", "fp64") else 8
+    """Device footprint of a resident operator, with a tenth of headroom: the factors
+    of every cell (whole blocks of nx x ny x ldn complex values in complex128; the
+    lower halves in 16 x 16 tiles, and the last whole inverse of each half chain, in
+    the reduced precisions), the per-problem vectors, the Krylov basis of a batch and
+    the sweeps' trace, output and scratch pools.  Every cell counts as an interior
+    one, the largest."""
+    dbl = precision in ("c128", "fp64")
+    cs = 16 if dbl else 8
+    cells = spec.N * spec.N
     side = spec.m + 6 + 2 * spec.p - 1          # interior cell DOFs per side (the largest)
-    ldn = (side + 3) // 4 * 4
-    factors = spec.N * spec.N * side * side * ldn * cs
+    if dbl:
+        factors = cells * side * side * ((side + 3) // 4 * 4) * cs
+    else:
+        rows = (side + 15) // 16
+        factors = cells * (side * rows * (rows + 1) // 2 * 256 + 2 * side * (side + 8)) * cs
     n2 = spec.n_dof * spec.n_dof
-    vectors = n2 * 8 + 16 * n2 * max_batch * (2 * (restart + 1) + 8) + 4 * cs * n2 * max_batch * 2
-    return int(1.25 * (factors + vectors))
+    vectors = n2 * 8 + 16 * n2 * max_batch * (2 * (restart + 1) + 8)
+    # pools: four output planes for up to two right-hand sides (a launch per sweep), one
+    # beyond; 24 trace lines per cell and shift; the lines of every slot of stage 1, or
+    # of eight sweeps' steps on several CTAs per half (twice the lines)
+    outs = 4 * n2 * cs * max(max_batch, 4 * min(max_batch, 2))
+    traces = max_batch * 4 * cells * 24 * ((side + 7) // 8 * 8) * cs
+    scratch = 4 * max_batch * (side + 1) * side * cs * max(cells, 16 * spec.N)
+    return int(1.1 * (factors + vectors + outs + traces + scratch))
 
 
 # ---------------------------------------------------------------------------
