@@ -14,7 +14,6 @@ built: no Eigen / libconfig++ / MPI)."""
 from __future__ import annotations
 
 import argparse
-import re
 import json
 import os
 import statistics
@@ -48,10 +47,18 @@ WORKLOAD = WORKLOADS["C4"]
 PRECISION = {"C1": "c64", "C2": "c64", "C3": "c64", "C4": "bf16x2"}
 DATA = {"C1": "synthetic (constant medium)", "C2": "synthetic (seeded Gaussian-lens medium)",
         "C3": "synthetic (seeded layered medium)", "C4": "synthetic (seeded piecewise-smooth random medium)"}
-# how L2 is kept out of the timing: every workload streams more factor bytes per apply than L2 holds
+# how L2 is kept out of the timing: C2 to C4 stream more factor bytes per apply than L2 holds;
+# C1's factors fit in L2, so a buffer larger than L2 is written before every timed solve (within
+# a solve they are read from L2 again)
+L2_FLUSH = {"C1"}
 L2_NOTE = {n: f"inputs larger than L2 (129 MB): {gb} of cell factors streamed per preconditioner apply"
-           for n, gb in (("C1", "0.14 GB with the Krylov basis"), ("C2", "1.2 GB (c64)"),
-                         ("C3", "5.6 GB (c64)"), ("C4", "23.9 GB (bf16x2)"))}
+           for n, gb in (("C2", "1.42 GB (c64)"), ("C3", "5.97 GB (c64)"), ("C4", "23.9 GB (bf16x2)"))}
+L2_NOTE["C1"] = ("L2 (129 MB) flushed before each timed solve (512 MB written); the 0.06 GB of cell factors (c64) "
+                 "fit in it and stay there during a solve")
+# DRAM bytes per algorithmic byte of a whole C2 apply, per-sweep launches, from an ncu capture of
+# the symmetric-tile sweep kernels (dram__bytes_read.sum + dram__bytes_write.sum over its launches);
+# batches that run one launch per step have no capture of these kernels
+TRAFFIC_PER_ALG_BYTE = {"c64": 0.967, "bf16x2": 0.962}
 DTYPE = {"c64": "c64 factors/applies + f64 Krylov",
          "bf16x2": "bf16-split factor products (hi+lo, fp32 accumulate) + f64 Krylov",
          "c128": "c128 factors/applies + f64 Krylov"}
@@ -304,12 +311,15 @@ def run_gpu(args):
     launches0 = S.info()["kernel_launches"]
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     reps = []
+    flush = torch.empty(1 << 29, dtype=torch.uint8, device=dev) if args.config.upper() in L2_FLUSH else None
     if dist:
         dist.barrier()
     torch.cuda.synchronize()
     with ClockSampler(local) as clk:
         t0 = time.perf_counter()
         for i in range(args.steps):
+            if flush is not None:
+                flush.fill_(i & 255)
             ev[i][0].record(st)
             _, rep = solve()
             ev[i][1].record(st)
@@ -336,6 +346,9 @@ def run_gpu(args):
     torch.cuda.synchronize()
     te = []
     for _ in range(args.e2e_steps):
+        if flush is not None:
+            flush.zero_()
+            torch.cuda.synchronize()
         t = time.perf_counter()
         xh, rep_h = S.solve_host(bnp, tol=args.tol, max_iter=300, restart=30, x_host=xnp)
         te.append(time.perf_counter() - t)
@@ -401,20 +414,11 @@ def run_gpu(args):
     achieved = pr["alg_bytes"] / (t_tuned_graph / 1e3) / 1e9
     achieved_sequential = pr["alg_bytes"] / (front_ms / 1e3) / 1e9
     peak, peak_kind = measured_peaks()
-    # DRAM traffic of the fronts: the ncu capture's traffic per algorithmic
-    # byte (a full C2 apply of the same kernel and precision) times this
+    # DRAM traffic of the fronts: the captured traffic per algorithmic byte times this
     # apply's algorithmic bytes
-    # (the capture of the same schedule kind: per-sweep launches or one launch
-    # per step, where one exists)
-    traffic, traffic_key = None, None
-    tf = ROOT / "profiles" / "k_front_dram_traffic.md"
-    if tf.exists() and prec in ("c64", "bf16x2"):
-        keys = ([prec + "_per_sweep"] if launch["per_sweep_launches"] else []) + [prec]
-        for key in keys:
-            m = re.search(r"traffic_per_alg_byte_%s:\s*([0-9.eE+]+)" % key, tf.read_text())
-            if m:
-                traffic, traffic_key = float(m.group(1)) * pr["alg_bytes"], key
-                break
+    traffic = None
+    if launch["per_sweep_launches"] and prec in TRAFFIC_PER_ALG_BYTE:
+        traffic = TRAFFIC_PER_ALG_BYTE[prec] * pr["alg_bytes"]
 
     # plain FP64 GPU path
     S64 = None
@@ -475,10 +479,11 @@ def run_gpu(args):
             if fp64 else None,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak if peak else None, "traffic": traffic,
-                         "traffic_source": "ncu DRAM bytes per algorithmic byte of a full C2 apply of this kernel "
-                                           "(traffic_per_alg_byte_%s in profiles/k_front_dram_traffic.md), times "
-                                           "this apply's algorithmic bytes" % traffic_key if traffic else None,
-                         "kernel": "k_front (sweep-front cell solves), all fronts of one apply (graph replay)",
+                         "traffic_source": "ncu DRAM bytes per algorithmic byte of a C2 apply of this kernel and "
+                                           "precision (%g), times this apply's algorithmic bytes"
+                                           % TRAFFIC_PER_ALG_BYTE[prec] if traffic else None,
+                         "kernel": "k_front%s (sweep-front cell solves), all fronts of one apply (graph replay)"
+                                   % ("" if prec == "c128" else "_sym"),
                          # the launches one by one on one stream (profiled): no overlap between
                          # launches, so below the replayed apply, far below with per-sweep launches
                          "achieved_launches_serialised": achieved_sequential,
