@@ -1146,7 +1146,8 @@ lsw_status lsw_ctx_create(lsw_ctx** out, int device) {
   if (const char* ev = std::getenv("LSW_SWEEP_LANES")) c->lanes_max_rhs = std::max(0, std::atoi(ev));
   // LSW_TUNE=0 leaves every sweep-front shape to the cost model
   if (const char* ev = std::getenv("LSW_TUNE")) c->tune = std::atoi(ev) != 0;
-  // LSW_SWEEP_TC=1 adds tensor-core line products to the complex64 tuning candidates
+  // LSW_SWEEP_TC=1 adds tensor-core line products to the complex64 tuning candidates; its
+  // factors are then whole blocks (sym_factors)
   if (const char* ev = std::getenv("LSW_SWEEP_TC")) c->sweep_tc = std::atoi(ev) != 0;
   // LSW_FRONT_SHAPE=RxC imposes R slots per item (1, 2, 4, 8, 16) and C CTAs per half
   // chain (1, 2, 4) on every sweep front where that shape fits (no tuning)
