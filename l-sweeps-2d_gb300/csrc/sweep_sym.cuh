@@ -31,12 +31,13 @@
 //   split:     mma.sync m16n8k16, the four products of hi and lo words against
 //              the input's hi and lo words, FP32 accumulation (the fourth, lo x
 //              lo, halves the preconditioner's error: 9e-5 against 2e-4 at 163-
-//              point cells).  Against whole blocks and three products a cell
-//              solve's error from the split is 0.72-0.87x; an apply's is 1.04-1.23x,
+//              point cells).  Against whole blocks and three products the split's
+//              own error is 0.72-0.87x in a cell solve and up to 1.23x in an apply,
 //              since the two entries that a value serves share its rounding and
-//              their errors add in what travels to and fro (against complex128
-//              1.04-1.18x at 33 to 64 points per line, 1.00x from 150 on, where the
-//              FP32 inverse dominates; mean of 16 media each).
+//              their errors add in what travels to and fro.  An apply's whole
+//              error against complex128 is 1.04x at 33 points per line, 1.18x at 54
+//              and 73, 1.06x at 129 and 1.00x from 163 on, where the FP32 inverse
+//              dominates (means over 16 media, +-0.01).
 // The partial sums go to every other CTA of the half (st.async into its shared
 // memory, completing the transaction count of its per-line mbarrier); each CTA
 // finishes every row, all in the same order, in the registers of the lanes
