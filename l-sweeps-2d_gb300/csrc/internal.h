@@ -64,7 +64,7 @@ struct DevCell {
 // the lower half of each line's inverse E^-1 S^-1 E as 16 x 16 tiles, tile
 // (I, J), I >= J, in class (I + J) mod 4; the classes in turn, each ordered by
 // column, then row.  complex64: element (i, j) of a tile at 16 j + (i ^ swz(j));
-// split: planes of 8 x 8 bf16 matrices (sym_put in kernels_factor.cu).
+// split: planes of 8 x 8 bf16 matrices (sym_put.cuh).
 constexpr int kSymTilesMax = 12;   // tile rows: 192 points per line
 struct SymTiles {
   static constexpr __host__ __device__ int rows(int ny) { return (ny + 15) >> 4; }
