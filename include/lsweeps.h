@@ -172,11 +172,12 @@ lsw_status lsw_ctx_set_graphs(lsw_ctx* ctx, int enable);
  * each item a thread-block cluster of 2 x `cluster` CTAs (the two half chains
  * of the cell's twisted block solve).  With tuning on (enable = 1, the default;
  * LSW_TUNE=0 in the environment at context creation turns it off) the first
- * apply of a batch size measures every shape (slots 4, 8, 16 x CTAs 1, 2, 4
- * per half) on every front where it fits, with CUDA events on the call's
- * stream, and keeps each front's fastest; the choice is cached per GPU (UUID)
- * and problem shape for the process, and appended to the file named by
- * LSW_TUNE_CACHE when that is set (read back by later processes).  With
+ * apply of a batch size measures every shape (slots 4, 8, 16, and 1 and 2 for
+ * fronts of few items, x CTAs 1, 2, 4 per half) on every kind of front where it
+ * fits, with CUDA events on the call's stream, and keeps each kind's fastest;
+ * the choice is cached per GPU (UUID) and problem shape for the process, and
+ * appended to the file named by LSW_TUNE_CACHE when that is set (read back by
+ * later processes that run the same kernels).  With
  * tuning off a cost model chooses.  Changing the setting drops the context's
  * schedules (rebuilt on next use; waits for the device).  No counterpart in the
  * reference (its sweeps are host loops, DDCheckerboard.cpp:812-880). */
@@ -191,12 +192,12 @@ lsw_status lsw_ctx_set_tuning(lsw_ctx* ctx, int enable);
  * and the sweeps fill the GPU between one another's launches; their outputs go
  * to one plane per stage-2 sweep, summed at the end (four times the output
  * pool of one launch per step).  Results equal those of one launch per step up
- * to the order of the final sums.  Their launch shapes come from the cost
- * model, with each launch assumed to share the GPU with 2, 4 or 8 others of
- * its size (launches timed alone do not show that sharing): with tuning on
- * (lsw_ctx_set_tuning) the first apply of a batch size times one whole apply
- * per assumption and keeps the fastest, cached like the per-front shapes;
- * with tuning off the assumption is 4.  Changing the setting drops the
+ * to the order of the final sums.  With tuning on
+ * (lsw_ctx_set_tuning) the first apply of a batch size times whole applies of
+ * up to six schedules (launches timed alone do not show how they share the GPU)
+ * and keeps the fastest, cached like the per-front shapes; with tuning off the
+ * cost model chooses, a launch taken to share the GPU with 4 of its size.
+ * Changing the setting drops the
  * context's schedules (rebuilt on next use; waits for the device).  No counterpart in the reference (its sweeps are host loops,
  * DDCheckerboard.cpp:812-880). */
 lsw_status lsw_ctx_set_sweep_lanes(lsw_ctx* ctx, int max_rhs);
